@@ -59,6 +59,33 @@ struct DevJob {
     int ttab;         // float2 offset of the twiddle tables of the job's radix plan
 };
 
+// Source of strip values in the self-contained job record of the four-strip
+// form (stage_quad.cuh): offsets at the job's first strip and the strip's (or
+// band's) first position.
+enum QSrcFlags : int {
+    QS_FIXED = 1,     // rigid domain: fields in the fixed buffer
+    QS_PML = 2,       // stale p0 at the first stage of a step
+    QS_NONE = 4,      // no neighbour: zero band
+    QS_ALIGNED = 8,   // column job whose strips start on a 16-byte boundary
+};
+struct alignas(16) QSrc {
+    long long oa, ob, op0;   // px or the velocity, py, the p0 array
+    int pitch, flags;
+};
+// One job of the four-strip form: everything a CTA needs besides the tables.
+struct alignas(16) QJob {
+    int L, kind, count, n;             // n: positions of a strip (pressure cells, or those + 1)
+    int W, scene, dom, dtab;
+    int wtab, ttab, pitch_out, att;    // att: PML profile of the updated field, -1 = none
+    float R1, T1, R2, T2;
+    long long o_out;                   // updated field at the job's first strip
+    float rho, c2;
+    float cdt[6];
+    float rinv;                        // 1 / rho, correctly rounded
+    int pad;
+    QSrc own, lo, hi;
+};
+
 struct DevReceiver {
     int dom, row, col;
 };

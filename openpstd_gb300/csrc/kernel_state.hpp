@@ -143,7 +143,7 @@ inline int planned_variant(int L) {
         for (int i = 0; sv && i < nv; i++) {
             const StageVariant& v = vs[i];
             if (v.CS == sv->CS && v.NT == sv->NT && v.smem == sv->smem && v.ctw == sv->ctw && v.shf == 0 &&
-                !v.persistent && !v.pipe && !v.bf16 && !v.tma && !v.tc5 && v.r[0] == sv->r[0] && v.r[1] == sv->r[1] &&
+                !v.persistent && !v.pipe && !v.bf16 && !v.tma && !v.tc5 && !v.quad && v.r[0] == sv->r[0] && v.r[1] == sv->r[1] &&
                 v.r[2] == sv->r[2] && v.r[3] == sv->r[3])
                 return i;
         }
@@ -168,6 +168,8 @@ struct PlanChoice {
     std::vector<std::pair<int, const StageVariant*>> vars;   // (L, variant)
     bool merged = false;
     int merged_fam = 0;
+    bool chained = false;
+    int chain_fam = 0;
     bool longest_first = false;
     std::string form;
 };
@@ -184,6 +186,7 @@ struct Bucket {
     int L = 0;
     const StageVariant* var = nullptr;
     int off = 0, n = 0;            // jobs in djobs
+    int qoff = 0;                  // first record in dqjobs (four-strip form)
     int tw_off = 0;                // float2 offset of the twiddles in dtw
     int fp_off = 0, fv_off = 0;    // float2 offsets of the pressure / velocity filters
     int rc = 4;                    // floats staged per strip by the pipelined form
@@ -217,6 +220,7 @@ struct Kernel {
 
     DevBuf<DevDomain> ddoms;
     DevBuf<DevJob> djobs;
+    DevBuf<QJob> dqjobs;              // records of the buckets whose variant is of the four-strip form
     DevBuf<float2> dfilt, dtw;
     DevBuf<float> dwin, datt;
     DevBuf<int> dpml;                 // indices of PML domains
@@ -330,10 +334,11 @@ struct Kernel {
     // same factors instead, extended to 2L + Q floats: hx[e] = h[(e - L) mod L].
     int filter_of(int L, bool vel, const StageVariant* v, float dxf) {
         const bool study = v->bf16 || v->tc5;
-        const int form = v->direct ? 8 + v->direct : study ? 3 : (v->shf ? 2 : 0) + (v->ctw ? 1 : 0) * 4;
+        const int form = v->direct ? 8 + v->direct : study ? 3 : (v->shf ? 2 : 0) + (v->ctw ? 1 : 0) * 4 + v->quad;
         auto key = std::make_tuple(L, (int)vel, v->r[0], v->r[1], v->r[2], v->r[3], dxf, form);
         auto it = filt_off.find(key);
         if (it != filt_off.end()) return it->second;
+        if (filt.size() & 1) filt.push_back(make_float2(0, 0));   // 16-byte loads
         int o = (int)filt.size();
         std::vector<std::complex<double>> gain(L, std::complex<double>(1, 0));
         if (!study && gain_compensation()) gain = tgain::round_trip_gain(L, v->r, v->np, v->ctw != 0, v->shf != 0);
@@ -373,7 +378,14 @@ struct Kernel {
             std::complex<double> c = full[j] / (double)L / gain[j];
             perm[pos[j]] = make_float2((float)c.real(), (float)c.imag());
         }
-        filt.insert(filt.end(), perm.begin(), perm.end());
+        if (v->quad) {   // pairs of the last pass's outputs, block after block: [R/2][L/R][2]
+            const int R = v->r[v->np - 1], B = L / R;
+            for (int h = 0; h < R / 2; h++)
+                for (int b = 0; b < B; b++)
+                    for (int e = 0; e < 2; e++) filt.push_back(perm[(size_t)b * R + 2 * h + e]);
+        } else {
+            filt.insert(filt.end(), perm.begin(), perm.end());
+        }
         filt_off[key] = o;
         return o;
     }
@@ -485,6 +497,64 @@ struct Kernel {
             }
         }
         return jobs;
+    }
+
+    // the self-contained record of a job (four-strip form), from its plan entry
+    // and the domain table
+    static QJob quad_job_of(const DevJob& j, const std::vector<DevDomain>& doms) {
+        QJob q;
+        std::memset(&q, 0, sizeof q);
+        q.att = -1;
+        q.kind = j.kind;
+        q.dom = j.dom;
+        q.own.flags = q.lo.flags = q.hi.flags = QS_NONE;
+        if (j.kind & JK_COPY) return q;
+        const bool vel = j.kind & JK_VEL, y = j.kind & JK_Y;
+        const DevDomain& d = doms[j.dom];
+        const int e = vel ? 1 : 0;
+        q.L = j.L;
+        q.count = j.count;
+        q.n = (y ? d.ny : d.nx) + e;
+        q.W = j.W;
+        q.scene = d.scene;
+        q.dtab = j.dtab;
+        q.wtab = j.wtab;
+        q.ttab = j.ttab;
+        q.R1 = j.R1; q.T1 = j.T1; q.R2 = j.R2; q.T2 = j.T2;
+        q.rho = d.rho;
+        q.c2 = d.c2;
+        q.rinv = 1.0f / d.rho;
+        for (int k = 0; k < 6; k++) q.cdt[k] = d.cdt[k];
+        // first strip s and position p of a source
+        auto source = [&](const DevDomain& f, int s, int p) {
+            QSrc r;
+            std::memset(&r, 0, sizeof r);
+            r.pitch = vel ? (y ? f.pitch_vy : f.pitch_vx) : f.pitch_p;
+            const long long at = y ? (long long)p * r.pitch + s : (long long)s * r.pitch + p;
+            r.oa = (vel ? (y ? f.o_vy : f.o_vx) : f.o_px) + at;
+            r.ob = f.o_py + at;
+            r.op0 = f.o_p0 + at;
+            r.flags = (f.fixed ? QS_FIXED : 0) | (f.pml ? QS_PML : 0) | (y && s % 4 == 0 ? QS_ALIGNED : 0);
+            return r;
+        };
+        q.own = source(d, j.first, 0);
+        if (j.d1 >= 0) q.lo = source(doms[j.d1], j.o1, (y ? doms[j.d1].ny : doms[j.d1].nx) - j.W);   // far end (vel: n1 - W - 1 of n1 = cells + 1)
+        if (j.d2 >= 0) q.hi = source(doms[j.d2], j.o2, e);
+        if (vel) {
+            q.pitch_out = d.pitch_p;
+            q.o_out = y ? d.o_py + j.first : d.o_px + (long long)j.first * d.pitch_p;
+        } else {
+            q.pitch_out = y ? d.pitch_vy : d.pitch_vx;
+            q.o_out = y ? d.o_vy + j.first : d.o_vx + (long long)j.first * d.pitch_vx;
+            q.att = y ? d.att_yv : d.att_xv;
+        }
+        return q;
+    }
+    static std::vector<QJob> quad_jobs_of(const std::vector<DevJob>& js, const std::vector<DevDomain>& doms) {
+        std::vector<QJob> out;
+        out.reserve(js.size());
+        for (const DevJob& j : js) out.push_back(quad_job_of(j, doms));
+        return out;
     }
 
     // ---------------------------------------------------------------- build
@@ -737,7 +807,8 @@ struct Kernel {
             side.push_back(s);
         }
         // the cache serves unforced plans only (PSTD_MERGED / PSTD_PLAN / PSTD_DFT pin choices)
-        const bool cacheable = autotune && !std::getenv("PSTD_MERGED") && !std::getenv("PSTD_PLAN") && !want_bf16_dft();
+        const bool cacheable = autotune && !std::getenv("PSTD_MERGED") && !std::getenv("PSTD_CHAIN") &&
+                               !std::getenv("PSTD_PLAN") && !want_bf16_dft();
         const std::string sig = cacheable ? plan_signature() : std::string();
         PlanChoice cached;
         bool hit = false;
@@ -759,6 +830,10 @@ struct Kernel {
                 merged = true;
                 capture_graphs();
             }
+            if (cached.chained) {
+                build_chain(cached.chain_fam);
+                chained = true;
+            }
             form_choice = cached.form + " (plan cache)";
         } else {
             plan(autotune);
@@ -774,6 +849,8 @@ struct Kernel {
                 pc.longest_first = longest_first;
                 pc.merged = merged;
                 pc.merged_fam = merged_fam;
+                pc.chained = chained;
+                pc.chain_fam = chain_fam;
                 pc.form = form_choice;
                 std::lock_guard<std::mutex> lock(plan_cache_mutex());
                 plan_cache()[sig] = pc;
@@ -921,6 +998,9 @@ struct Kernel {
                     DevBuf<DevJob> tj;
                     tj.upload(all[i]);
                     StageArgs a = stage_args(cur, 1, tj.p, dtw.p + twv[i], fpv[i], fvv[i], b.rc);
+                    DevBuf<QJob> tq;
+                    if (vs[i].quad) tq.upload(quad_jobs_of(all[i], hdoms));
+                    a.qjobs = tq.p;
                     if (vs[i].launch((int)all[i].size(), a, stream) != cudaSuccess) {
                         cudaGetLastError();   // this variant's staging does not fit the bucket's strips
                         rec += " " + std::to_string(i) + ":n/a";
@@ -956,6 +1036,7 @@ struct Kernel {
             }
         }
         std::vector<DevJob> jobs;
+        std::vector<QJob> qjobs;
         for (size_t i = 0; i < buckets.size(); i++) {
             auto& b = buckets[i];
             auto js = make_jobs(b.L, b.var, i + 1 == buckets.size());
@@ -974,9 +1055,15 @@ struct Kernel {
             b.off = (int)jobs.size();
             b.n = (int)js.size();
             jobs.insert(jobs.end(), js.begin(), js.end());
+            b.qoff = (int)qjobs.size();
+            if (b.var->quad) {
+                auto qs = quad_jobs_of(js, hdoms);
+                qjobs.insert(qjobs.end(), qs.begin(), qs.end());
+            }
         }
         upload_tables();
         djobs.upload(jobs);
+        dqjobs.upload(qjobs);
     }
 
     void reset() {
@@ -992,7 +1079,69 @@ struct Kernel {
         steps = 0;
     }
 
-    int launches_per_step() const { return 6 * (int)stage_launches().size() + (n_pml > 0 || dev_counts) + 1; }
+    int launches_per_step() const {
+        if (chained) return 7 + (spectral ? 2 : 0);
+        return 6 * (int)stage_launches().size() + (n_pml > 0 || dev_counts) + 1;
+    }
+
+    // ---------------------------------------------------------------- chained form
+    // One launch per RK stage over all lengths and one after them
+    // (stage_chain.cu); chosen at create time when it is faster on the scene's
+    // own steps.
+    bool chained = false;
+    int chain_fam = 0;
+    int n_chain = 0;
+    size_t chain_smem = 0;
+    DevBuf<QJob> dqjobs_chain;
+
+    bool any_pinned() const {
+        for (const Bucket& b : buckets)
+            if (b.pinned) return true;
+        return false;
+    }
+
+    // records of every length, longest transform first, then the copy jobs
+    void build_chain(int fam) {
+        chain_fam = fam;
+        std::vector<DevJob> all;
+        chain_smem = 0;
+        for (size_t i = buckets.size(); i-- > 0;) {
+            const StageVariant* v = chain_variant(buckets[i].L, fam);
+            auto js = make_jobs(buckets[i].L, v, false);
+            all.insert(all.end(), js.begin(), js.end());
+            chain_smem = std::max(chain_smem, (size_t)v->smem);
+        }
+        auto copies = make_jobs(-1, chain_variant(128, fam), true);   // no strips of length -1: the copy jobs only
+        all.insert(all.end(), copies.begin(), copies.end());
+        n_chain = (int)all.size();
+        dqjobs_chain.upload(quad_jobs_of(all, hdoms));
+        CK(prepare_chain(fam));
+        upload_tables();
+    }
+
+    void enqueue_chain_step(int c, cudaStream_t st, std::vector<std::pair<cudaEvent_t, cudaEvent_t>>* ev) {
+        const int B = (c + 2) % 3;
+        for (int k = 0; k < 6; k++) {
+            cudaEvent_t t0 = nullptr, t1 = nullptr;
+            if (ev) {
+                CK(cudaEventCreate(&t0));
+                CK(cudaEventCreate(&t1));
+                CK(cudaEventRecord(t0, st));
+            }
+            StageArgs a = stage_args(c, k, nullptr, dtw.p, 0, 0, 0);
+            a.qjobs = dqjobs_chain.p;
+            CK(launch_chain(chain_fam, n_chain, a, chain_smem, st));
+            if (ev) {
+                CK(cudaEventRecord(t1, st));
+                ev->push_back({t0, t1});
+            }
+        }
+        CK(launch_step_post(dpml.p, n_pml, dpml_off.p, pml_blocks, ddoms.p, sets[B].p, fixed.p, p0.p, datt.p, drec.p, n_rec,
+                            spectral ? nullptr : dring.p, ring_cap, dcounter.p, first_step.p, (int)scenes.size(), st));
+        if (spectral)
+            CK(launch_spectral_receivers(dsi_rows.p, n_si_rows, dsi_w.p, dsi_first.p, n_rec, ddoms.p, sets[B].p, fixed.p,
+                                         p0.p, dsi_val.p, dring.p, ring_cap, dcounter.p, st));
+    }
 
     // ---------------------------------------------------------------- merged form
     // One persistent launch per RK stage over the jobs of every length the
@@ -1005,6 +1154,7 @@ struct Kernel {
         bool all;
         const int* cnt = nullptr;   // device-count persistent launch (launch_dev): its job count
         int ctr = 0;                // and its job counter (counters[stage * 16 + ctr])
+        const QJob* qjobs = nullptr;   // four-strip form: its records
     };
     // serving form, one persistent launch per strip length: the configuration,
     // first job in djobs_all, index of the job count in dev_counts, twiddles
@@ -1020,6 +1170,7 @@ struct Kernel {
     int merged_fam = merged_family_default();   // configuration family of the merged launch
     bool longest_first = false;   // launch order of the lengths in a stage (buckets ascend in L)
     DevBuf<DevJob> djobs_all, djobs_sep;
+    DevBuf<QJob> dqjobs_sep;
     int n_all = 0;
     std::vector<SepBucket> sep;
     DevBuf<int> counters;
@@ -1044,10 +1195,13 @@ struct Kernel {
             if (n_all > 0 || dev_counts) v.push_back({nullptr, djobs_all.p, n_all, 0, 0, 0, 0, true});
             for (const SepBucket& q : sep) {
                 const Bucket& b = buckets[q.b];
-                v.push_back({b.var, djobs_sep.p + q.off, q.n, b.tw_off, b.fp_off, b.fv_off, b.rc, false});
+                v.push_back({b.var, djobs_sep.p + q.off, q.n, b.tw_off, b.fp_off, b.fv_off, b.rc, false, nullptr, 0,
+                             dqjobs_sep.p + q.off});
             }
         } else {
-            for (const Bucket& b : buckets) v.push_back({b.var, djobs.p + b.off, b.n, b.tw_off, b.fp_off, b.fv_off, b.rc, false});
+            for (const Bucket& b : buckets)
+                v.push_back({b.var, djobs.p + b.off, b.n, b.tw_off, b.fp_off, b.fv_off, b.rc, false, nullptr, 0,
+                             dqjobs.p + b.qoff});
             if (longest_first) std::reverse(v.begin(), v.end());
         }
         return v;
@@ -1083,6 +1237,7 @@ struct Kernel {
         n_all = (int)all.size();
         djobs_all.upload(all);
         djobs_sep.upload(rest);
+        dqjobs_sep.upload(quad_jobs_of(rest, hdoms));
         counters.alloc(6);
         CK(prepare_stage_all(merged_fam));
         upload_tables();
@@ -1167,7 +1322,15 @@ struct Kernel {
     void choose_form(bool tune) {
         int force = -1;
         if (const char* e = std::getenv("PSTD_MERGED")) force = std::atoi(e) != 0;
-        if (!any_mergeable() || force == 0 || (force < 0 && !tune)) {
+        chained = false;
+        if (const char* e = std::getenv("PSTD_CHAIN"); e && force < 0 && !any_pinned()) {   // 0 / 1: that family
+            build_chain(std::atoi(e) == 1 ? 1 : 0);
+            merged = false;
+            chained = true;
+            form_choice = "chained launches (forced), family " + std::to_string(chain_fam);
+            return;
+        }
+        if ((!any_mergeable() && (any_pinned() || force == 1)) || force == 0 || (force < 0 && !tune)) {
             merged = false;
             form_choice = "per-length launches";
             return;
@@ -1183,6 +1346,23 @@ struct Kernel {
         capture_graphs();
         const float t_len = time_steps(5);
         reset();
+        // both families of the chained form
+        float t_chain = 1e30f;
+        int best_chain = 0;
+        std::string crec;
+        for (int f = 0; f < 2 && !any_pinned(); f++) {
+            build_chain(f);
+            chained = true;
+            capture_graphs();
+            const float t = time_steps(5);
+            reset();
+            chained = false;
+            char b[64];
+            std::snprintf(b, sizeof b, "%s%.1f us family %d", f ? ", " : " (step chained ", t * 1e3f, f);
+            crec += b;
+            if (t < t_chain) { t_chain = t; best_chain = f; }
+        }
+        if (!crec.empty()) crec += ")";
         // both configuration families of the merged launch (PSTD_MERGED_FAMILY: that one only)
         std::vector<int> fams{0, 1};
         if (std::getenv("PSTD_MERGED_FAMILY")) fams.assign(1, merged_family_default());
@@ -1190,6 +1370,7 @@ struct Kernel {
         int best_fam = fams[0];
         std::string rec;
         for (int f : fams) {
+            if (!any_mergeable()) break;
             merged_fam = f;
             build_merged();
             merged = true;
@@ -1201,18 +1382,25 @@ struct Kernel {
             rec += b;
             if (t < t_all) { t_all = t; best_fam = f; }
         }
-        char buf[200];
+        char buf[400];
         std::snprintf(buf, sizeof buf, " (step merged %s vs %.1f us per length)", rec.c_str(), t_len * 1e3f);
+        merged = false;
+        if (t_chain < t_len && t_chain < t_all) {
+            build_chain(best_chain);
+            chained = true;
+            capture_graphs();
+            form_choice = "chained launches, family " + std::to_string(best_chain) + buf + crec;
+            return;
+        }
+        std::strncat(buf, crec.c_str(), sizeof buf - std::strlen(buf) - 1);
         if (t_all >= t_len) {
-            merged = false;
             capture_graphs();
             form_choice = std::string("per-length launches") + buf;
         } else {
-            if (merged_fam != best_fam) {
-                merged_fam = best_fam;
-                build_merged();
-                capture_graphs();
-            }
+            merged = true;
+            merged_fam = best_fam;
+            build_merged();
+            capture_graphs();
             form_choice = std::string("merged launch, family ") + std::to_string(best_fam) + buf;
         }
     }
@@ -1222,6 +1410,7 @@ struct Kernel {
     // each stage's launches, which then run back to back on `st`.
     void enqueue_step(int c, cudaStream_t st, bool concurrent,
                       std::vector<std::pair<cudaEvent_t, cudaEvent_t>>* ev = nullptr) {
+        if (chained) return enqueue_chain_step(c, st, ev);
         const int B = (c + 2) % 3;
         std::vector<cudaEvent_t> tmp;
         auto mk = [&]() {
@@ -1250,6 +1439,7 @@ struct Kernel {
                     CK(launch_stage_all(merged_fam, l.n, stage_args(c, k, l.jobs, dtw.p, 0, 0, 0), counters.p + k, s));
                 } else {
                     StageArgs a = stage_args(c, k, l.jobs, dtw.p + l.tw_off, l.fp, l.fv, l.rc);
+                    a.qjobs = l.qjobs;
                     CK(l.var->launch(l.n, a, s));
                 }
             };

@@ -36,6 +36,7 @@ struct StageArgs {
     // job of a scene that has taken all its steps is skipped (null: none skip)
     const int* scene_step = nullptr;
     const int* scene_limit = nullptr;
+    const QJob* qjobs = nullptr;   // four-strip form: its jobs
 };
 
 constexpr int PSTD_TMAP_BYTES = 128;   // sizeof(CUtensorMap)
@@ -62,6 +63,7 @@ struct StageVariant {
     bool tma = false;                                           // staged form: needs tensor maps and a row cap
     int ctw = 0;                                                // twiddle tables hold powers (Cfg::CTW)
     bool tc5 = false;                                           // tcgen05 TF32x3 DFT (precision study, opt-in)
+    int quad = 0;                                               // four-strip form: jobs are QJob records
     int direct = 0;                                             // direct convolution, Q outputs per task (filter: h)
     cudaError_t (*launch)(int n_jobs, const StageArgs& a, cudaStream_t st);
     cudaError_t (*prepare)();
@@ -98,6 +100,18 @@ cudaError_t launch_stage_all_dev(int fam, const int* counts, const StageArgs& a,
 // configuration per transform length 32..8192 with launch_dev set (nullptr
 // for other lengths)
 const StageVariant* serve_variant(int L);
+
+// chained form (stage_chain.cu): one launch per RK stage over the QJob records
+// of every length, programmatic stream serialisation; family 0 or 1.  smem:
+// the largest StageVariant::smem of the lengths present.
+const StageVariant* chain_variant(int L, int fam);
+cudaError_t prepare_chain(int fam);
+cudaError_t launch_chain(int fam, int n_jobs, const StageArgs& a, size_t smem, cudaStream_t st);
+// the PML multiply, receiver samples (ring == nullptr: none), step counter and
+// first-step flags of the chained form in one launch
+cudaError_t launch_step_post(const int* idx, int n_pml, const int* off, int pml_blocks, const DevDomain* doms, float* set,
+                             float* fixed, float* p0, const float* att, const DevReceiver* rec, int n_rec, float* ring,
+                             int ring_cap, int* counter, int* first_step, int n_scenes, cudaStream_t st);
 
 // one block per (row, 128-column chunk): with off (n + 1 prefix sums of the
 // domains' (rows + 1) x ceil((columns + 1) / 128) block counts) blocks is their

@@ -5,6 +5,7 @@
 #include <vector>
 
 #include "launch.hpp"
+#include "pml_post.cuh"
 
 namespace pstd {
 
@@ -25,6 +26,13 @@ const StageVariant* stage_variants_toeplitz_ws(int L, int* n);
 const StageVariant* stage_variants_tma_a(int L, int* n);
 const StageVariant* stage_variants_tma_b(int L, int* n);
 
+const StageVariant* stage_variants_quad_a(int L, int* n);
+const StageVariant* stage_variants_quad_b(int L, int* n);
+
+static const StageVariant* stage_variants_quad(int L, int* n) {
+    return L <= 512 ? stage_variants_quad_a(L, n) : stage_variants_quad_b(L, n);
+}
+
 static const StageVariant* stage_variants_tma(int L, int* n) {
     if (L <= 512) return stage_variants_tma_a(L, n);
     return stage_variants_tma_b(L, n);
@@ -40,7 +48,9 @@ static const StageVariant* stage_variants_fused(int L, int* n) {
 // Per length: the fused-form variants first (the default when nothing is
 // tuned), then the TMA-staged persistent forms, then the split gather /
 // transform / epilogue forms, then the precision-study variants, then the
-// direct-convolution forms of short strips (CUDA cores, then tcgen05).  Built once, before any launch.
+// direct-convolution forms of short strips (CUDA cores, then tcgen05), then the
+// four-strip forms (lengths with study variants: before those, which stay
+// last).  Built once, before any launch.
 int stage_variants(int L, const StageVariant** out) {
     static const std::vector<std::vector<StageVariant>> lists = [] {
         std::vector<std::vector<StageVariant>> all(14);
@@ -56,14 +66,21 @@ int stage_variants(int L, const StageVariant** out) {
             else v = stage_variants_huge(len, &n);
             for (int i = 0; i < nf; i++) all[lg].push_back(f[i]);
             for (int i = 0; i < nt; i++) all[lg].push_back(tv[i]);
-            for (int i = 0; i < n; i++) all[lg].push_back(v[i]);
-            int nd = 0;
+            int nd = 0, nq = 0, i = 0;
+            const StageVariant* qv = stage_variants_quad(len, &nq);
+            while (i < n && !v[i].bf16) all[lg].push_back(v[i++]);
+            if (i < n) {   // the precision-study variants come last in their lists
+                for (int q = 0; q < nq; q++) all[lg].push_back(qv[q]);
+                nq = 0;
+            }
+            while (i < n) all[lg].push_back(v[i++]);
             const StageVariant* dv = stage_variants_direct(len, &nd);
             for (int i = 0; i < nd; i++) all[lg].push_back(dv[i]);
             const StageVariant* ev = stage_variants_toeplitz(len, &nd);
             for (int i = 0; i < nd; i++) all[lg].push_back(ev[i]);
             const StageVariant* wv = stage_variants_toeplitz_ws(len, &nd);
             for (int i = 0; i < nd; i++) all[lg].push_back(wv[i]);
+            for (int q = 0; q < nq; q++) all[lg].push_back(qv[q]);
         }
         return all;
     }();
@@ -75,48 +92,6 @@ int stage_variants(int L, const StageVariant** out) {
     if (v.empty()) return 0;
     *out = v.data();
     return (int)v.size();
-}
-
-// After the sixth stage, for every PML domain (kernel/Solver.cpp:85,
-// kernel/core/Domain.cpp:716-725): keep p0 = px + py from before the multiply
-// (the reference does not recompute p0 after it), then px *= ax, py *= ay.
-// vx and vy of non-rigid domains were attenuated in the stage epilogue; rigid
-// domains (fields in the fixed buffer) get all four multiplies here.
-// one (row, 128-column chunk) block `lb` of PML domain doms[idx[dj]]
-__device__ __forceinline__ void pml_post_block(int dj, int lb, const int* idx, const DevDomain* doms, float* set,
-                                               float* fixed, float* p0, const float* __restrict__ att) {
-    const DevDomain d = doms[idx[dj]];
-    float* base = d.fixed ? fixed : set;
-    const int chunks = (d.nx + 1 + 127) >> 7;   // vx rows have nx + 1 columns
-    const int r = lb / chunks, i = ((lb - r * chunks) << 7) + threadIdx.x;
-    if (r < d.ny && i < d.nx) {
-        const long long e = (long long)r * d.pitch_p + i;
-        const float px = base[d.o_px + e], py = base[d.o_py + e];
-        p0[d.o_p0 + e] = __fadd_rn(px, py);
-        if (d.att_xp >= 0) base[d.o_px + e] = __fmul_rn(px, att[d.att_xp + i]);
-        if (d.att_yp >= 0) base[d.o_py + e] = __fmul_rn(py, att[d.att_yp + r]);
-    }
-    if (d.fixed) {
-        if (r < d.ny && i < d.nx + 1 && d.att_xv >= 0) {
-            const long long e = d.o_vx + (long long)r * d.pitch_vx + i;
-            base[e] = __fmul_rn(base[e], att[d.att_xv + i]);
-        }
-        if (r < d.ny + 1 && i < d.nx && d.att_yv >= 0) {
-            const long long e = d.o_vy + (long long)r * d.pitch_vy + i;
-            base[e] = __fmul_rn(base[e], att[d.att_yv + r]);
-        }
-    }
-}
-
-// the domain of flat block b: the last k with off[k] <= b (off ascends, off[0] = 0)
-__device__ __forceinline__ int pml_domain_of(const int* off, int n, int b) {
-    int lo = 0, hi = n - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (off[mid] <= b) lo = mid;
-        else hi = mid - 1;
-    }
-    return lo;
 }
 
 __global__ void pml_post_kernel(const int* idx, int n, const int* off, const DevDomain* doms, float* set,
