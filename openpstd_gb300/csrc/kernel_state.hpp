@@ -265,6 +265,8 @@ struct Kernel {
     DevBuf<long long> dframe_off;
     // run()'s frame slots (device) and their pinned host staging, kept across
     // runs; made at create for frames of up to 8 slots in 128 MiB
+    DevBuf<float> snap;      // dense p0 of a snapshot
+    std::mutex snap_mu;
     PinnedBuf run_stage;
     DevBuf<float> run_slots;
     // frames in flight of run() for slots of `slot` floats: up to 8 within 64 MiB, at least 3

@@ -143,6 +143,8 @@ cudaError_t launch_server_receivers(const DevSrvReceiver* rec, int n_rec, const 
                                     float* aux, int* scene_step, const int* scene_limit, const int* slots, int n_slots,
                                     cudaStream_t st, const int* counts = nullptr);
 // dense p0 = px + py of the given domains into dst (frames); sub > 1 keeps
+// dense p0 = px + py of one domain
+cudaError_t launch_field_sum(const float* px, const float* py, int pitch, int rows, int cols, float* dst, cudaStream_t st);
 // every sub-th row and column (ceil(nx/sub) x ceil(ny/sub) values per domain);
 // n_rec floats of rec_src (a receiver row) are copied to rec_dst on the way
 cudaError_t launch_frame(const int* doms_idx, const long long* dst_off, int n, const DevDomain* doms, const float* set,

@@ -279,6 +279,21 @@ cudaError_t launch_pml_post(const int* idx, int n, int blocks, const DevDomain* 
     return cudaGetLastError();
 }
 
+// dense p0 = px + py of one domain (snapshots)
+__global__ void field_sum_kernel(const float* __restrict__ px, const float* __restrict__ py, int pitch, int rows, int cols,
+                                 float* __restrict__ dst) {
+    for (int r = blockIdx.x; r < rows; r += gridDim.x)
+        for (int i = threadIdx.x; i < cols; i += blockDim.x) {
+            const long long e = (long long)r * pitch + i;
+            dst[(long long)r * cols + i] = __fadd_rn(px[e], py[e]);
+        }
+}
+
+cudaError_t launch_field_sum(const float* px, const float* py, int pitch, int rows, int cols, float* dst, cudaStream_t st) {
+    field_sum_kernel<<<std::min(rows, 2048), 256, 0, st>>>(px, py, pitch, rows, cols, dst);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_pml_post_dev(const int* idx, const int* counts, const int* off, const DevDomain* doms, float* set,
                                 float* fixed, float* p0, const float* att, const int* scene_step,
                                 const int* scene_limit, cudaStream_t st) {

@@ -356,10 +356,13 @@ int pstd_get_receivers(pstd_kernel* h, int32_t first_step, int32_t n_steps, floa
     if (k->n_rec == 0 || n_steps == 0) return PSTD_OK;
     GUARD({
         CK(cudaDeviceSynchronize());
-        for (int s = 0; s < n_steps; s++) {
-            int row = (first_step + s) % k->ring_cap;
-            CK(cudaMemcpy(dst + (size_t)s * k->n_rec, k->dring.p + (size_t)row * k->n_rec, k->n_rec * sizeof(float),
-                          cudaMemcpyDeviceToHost));
+        // the ring's rows are contiguous: at most one wrap
+        for (int s = 0; s < n_steps;) {
+            const int row = (first_step + s) % k->ring_cap;
+            const int n = std::min(n_steps - s, k->ring_cap - row);
+            CK(cudaMemcpy(dst + (size_t)s * k->n_rec, k->dring.p + (size_t)row * k->n_rec,
+                          (size_t)n * k->n_rec * sizeof(float), cudaMemcpyDeviceToHost));
+            s += n;
         }
         return PSTD_OK;
     })
@@ -391,12 +394,31 @@ int pstd_snapshot(pstd_kernel* h, int32_t idx, int32_t field, float* dst, int64_
                 CK(cudaMemcpy2D(dst, cols * sizeof(float), k->p0.p + d.o_p0, pitch * sizeof(float), cols * sizeof(float),
                                 rows, cudaMemcpyDeviceToHost));
             } else {
-                std::vector<float> a((size_t)rows * cols), b((size_t)rows * cols);
-                CK(cudaMemcpy2D(a.data(), cols * sizeof(float), base + d.o_px, pitch * sizeof(float), cols * sizeof(float),
-                                rows, cudaMemcpyDeviceToHost));
-                CK(cudaMemcpy2D(b.data(), cols * sizeof(float), base + d.o_py, pitch * sizeof(float), cols * sizeof(float),
-                                rows, cudaMemcpyDeviceToHost));
-                for (size_t i = 0; i < a.size(); i++) dst[i] = a[i] + b[i];
+                // summed on the device in blocks of rows, one contiguous copy
+                // each; the buffer (at most 64 MiB) is the handle's, callers may overlap
+                std::lock_guard<std::mutex> lock(k->snap_mu);
+                const int step = std::max(1, std::min(rows, (16 << 20) / std::max(cols, 1)));
+                const size_t m = (size_t)step * cols;
+                if (k->snap.n < m) {
+                    k->snap.release();
+                    if (cudaMalloc(&k->snap.p, m * sizeof(float)) == cudaSuccess) k->snap.n = m;
+                    else k->snap.p = nullptr, cudaGetLastError();
+                }
+                for (int r = 0; r < rows && k->snap.p; r += step) {
+                    const int nr = std::min(step, rows - r);
+                    const long long e = (long long)r * pitch;
+                    CK(launch_field_sum(base + d.o_px + e, base + d.o_py + e, pitch, nr, cols, k->snap.p, k->stream));
+                    CK(cudaStreamSynchronize(k->stream));
+                    CK(cudaMemcpy(dst + (size_t)r * cols, k->snap.p, (size_t)nr * cols * sizeof(float), cudaMemcpyDeviceToHost));
+                }
+                if (!k->snap.p) {   // no device memory left: sum on the host
+                    std::vector<float> b((size_t)rows * cols);
+                    CK(cudaMemcpy2D(dst, cols * sizeof(float), base + d.o_px, pitch * sizeof(float), cols * sizeof(float),
+                                    rows, cudaMemcpyDeviceToHost));
+                    CK(cudaMemcpy2D(b.data(), cols * sizeof(float), base + d.o_py, pitch * sizeof(float),
+                                    cols * sizeof(float), rows, cudaMemcpyDeviceToHost));
+                    for (size_t i = 0; i < b.size(); i++) dst[i] += b[i];
+                }
             }
         } else {
             CK(cudaMemcpy2D(dst, cols * sizeof(float), base + o, pitch * sizeof(float), cols * sizeof(float), rows,
@@ -697,7 +719,7 @@ static int solve_noalloc(const pstd_config* config, int n_steps, float* frame_de
         const int nv = stage_variants(b.L, &vs);
         // one CTA per job, no staging row cap, FP32 arithmetic
         for (int q = 0; q < nv && !b.var; q++)
-            if (!vs[q].persistent && !vs[q].pipe && !vs[q].bf16 && !vs[q].tma) b.var = &vs[q];
+            if (!vs[q].persistent && !vs[q].pipe && !vs[q].bf16 && !vs[q].tma && !vs[q].quad) b.var = &vs[q];
         if (!b.var)
             return fail(PSTD_ERR_UNSUPPORTED, "strip transform length " + std::to_string(b.L) +
                                                   " is outside the compiled range 32..8192");
