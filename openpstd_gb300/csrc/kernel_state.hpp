@@ -143,7 +143,7 @@ inline int planned_variant(int L) {
         for (int i = 0; sv && i < nv; i++) {
             const StageVariant& v = vs[i];
             if (v.CS == sv->CS && v.NT == sv->NT && v.smem == sv->smem && v.ctw == sv->ctw && v.shf == 0 &&
-                !v.persistent && !v.pipe && !v.bf16 && !v.tma && !v.tc5 && !v.quad && v.r[0] == sv->r[0] && v.r[1] == sv->r[1] &&
+                !v.persistent && !v.pipe && !v.bf16 && !v.tma && !v.tc5 && v.quad == sv->quad && v.r[0] == sv->r[0] && v.r[1] == sv->r[1] &&
                 v.r[2] == sv->r[2] && v.r[3] == sv->r[3])
                 return i;
         }
@@ -1155,7 +1155,6 @@ struct Kernel {
         int n, tw_off, fp, fv, rc;
         bool all;
         const int* cnt = nullptr;   // device-count persistent launch (launch_dev): its job count
-        int ctr = 0;                // and its job counter (counters[stage * 16 + ctr])
         const QJob* qjobs = nullptr;   // four-strip form: its records
     };
     // serving form, one persistent launch per strip length: the configuration,
@@ -1173,6 +1172,7 @@ struct Kernel {
     bool longest_first = false;   // launch order of the lengths in a stage (buckets ascend in L)
     DevBuf<DevJob> djobs_all, djobs_sep;
     DevBuf<QJob> dqjobs_sep;
+    DevBuf<QJob> dqjobs_all;   // serving loop: the records of djobs_all's entries (four-strip configurations)
     int n_all = 0;
     std::vector<SepBucket> sep;
     DevBuf<int> counters;
@@ -1190,19 +1190,19 @@ struct Kernel {
                 const DevRegion& g = dev_regions[r];
                 StageLaunch l{g.var, djobs_all.p + g.base, 0, g.tw_off, 0, 0, 0, false};
                 l.cnt = dev_counts + g.count_idx;
-                l.ctr = (int)r;
+                l.qjobs = dqjobs_all.p + g.base;
                 v.push_back(l);
             }
         } else if (merged) {
             if (n_all > 0 || dev_counts) v.push_back({nullptr, djobs_all.p, n_all, 0, 0, 0, 0, true});
             for (const SepBucket& q : sep) {
                 const Bucket& b = buckets[q.b];
-                v.push_back({b.var, djobs_sep.p + q.off, q.n, b.tw_off, b.fp_off, b.fv_off, b.rc, false, nullptr, 0,
+                v.push_back({b.var, djobs_sep.p + q.off, q.n, b.tw_off, b.fp_off, b.fv_off, b.rc, false, nullptr,
                              dqjobs_sep.p + q.off});
             }
         } else {
             for (const Bucket& b : buckets)
-                v.push_back({b.var, djobs.p + b.off, b.n, b.tw_off, b.fp_off, b.fv_off, b.rc, false, nullptr, 0,
+                v.push_back({b.var, djobs.p + b.off, b.n, b.tw_off, b.fp_off, b.fv_off, b.rc, false, nullptr,
                              dqjobs.p + b.qoff});
             if (longest_first) std::reverse(v.begin(), v.end());
         }
@@ -1325,8 +1325,8 @@ struct Kernel {
         int force = -1;
         if (const char* e = std::getenv("PSTD_MERGED")) force = std::atoi(e) != 0;
         chained = false;
-        if (const char* e = std::getenv("PSTD_CHAIN"); e && force < 0 && !any_pinned()) {   // 0 / 1: that family
-            build_chain(std::atoi(e) == 1 ? 1 : 0);
+        if (const char* e = std::getenv("PSTD_CHAIN"); e && force < 0 && !any_pinned()) {   // that family
+            build_chain(std::min(std::max(std::atoi(e), 0), CHAIN_FAMILIES - 1));
             merged = false;
             chained = true;
             form_choice = "chained launches (forced), family " + std::to_string(chain_fam);
@@ -1348,11 +1348,11 @@ struct Kernel {
         capture_graphs();
         const float t_len = time_steps(5);
         reset();
-        // both families of the chained form
+        // the families of the chained form
         float t_chain = 1e30f;
         int best_chain = 0;
         std::string crec;
-        for (int f = 0; f < 2 && !any_pinned(); f++) {
+        for (int f = 0; f < CHAIN_FAMILIES && !any_pinned(); f++) {
             build_chain(f);
             chained = true;
             capture_graphs();
@@ -1421,7 +1421,7 @@ struct Kernel {
             tmp.push_back(e);
             return e;
         };
-        if (merged) CK(cudaMemsetAsync(counters.p, 0, counters.n * sizeof(int), st));   // per-stage job counters
+        if (merged && dev_regions.empty()) CK(cudaMemsetAsync(counters.p, 0, counters.n * sizeof(int), st));   // per-stage job counters
         for (int k = 0; k < 6; k++) {
             cudaEvent_t t0 = nullptr, t1 = nullptr;
             if (ev) {
@@ -1433,7 +1433,8 @@ struct Kernel {
             auto launch = [&](const StageLaunch& l, cudaStream_t s) {
                 if (l.cnt) {
                     StageArgs a = stage_args(c, k, l.jobs, dtw.p + l.tw_off, 0, 0, 0);
-                    CK(l.var->launch_dev(l.cnt, a, counters.p + k * 16 + l.ctr, s));
+                    a.qjobs = l.qjobs;
+                    CK(l.var->launch_dev(l.cnt, a, s));
                 } else if (l.all && dev_counts) {
                     CK(launch_stage_all_dev(merged_fam, dev_counts, stage_args(c, k, l.jobs, dtw.p, 0, 0, 0),
                                             counters.p + k, s));

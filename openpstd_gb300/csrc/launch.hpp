@@ -69,11 +69,11 @@ struct StageVariant {
     cudaError_t (*prepare)();
     size_t (*smem_for)(int row_cap);                            // dynamic shared memory of one CTA
     const char* name;
-    // persistent form over a job table whose length is read from device
-    // memory at launch time (serving loop; null where not compiled): resident
-    // CTAs take jobs from *counter, skip all-zero jobs and jobs of scenes at
+    // persistent form over a table of QJob records whose length is read from
+    // device memory at launch time (serving loop; null where not compiled):
+    // resident CTAs stride over it, skip all-zero entries and jobs of scenes at
     // their step limit
-    cudaError_t (*launch_dev)(const int* count, const StageArgs& a, int* counter, cudaStream_t st) = nullptr;
+    cudaError_t (*launch_dev)(const int* count, const StageArgs& a, cudaStream_t st) = nullptr;
     cudaError_t (*prepare_dev)() = nullptr;
 };
 
@@ -102,8 +102,9 @@ cudaError_t launch_stage_all_dev(int fam, const int* counts, const StageArgs& a,
 const StageVariant* serve_variant(int L);
 
 // chained form (stage_chain.cu): one launch per RK stage over the QJob records
-// of every length, programmatic stream serialisation; family 0 or 1.  smem:
+// of every length, programmatic stream serialisation; family 0 .. 2.  smem:
 // the largest StageVariant::smem of the lengths present.
+constexpr int CHAIN_FAMILIES = 3;
 const StageVariant* chain_variant(int L, int fam);
 cudaError_t prepare_chain(int fam);
 cudaError_t launch_chain(int fam, int n_jobs, const StageArgs& a, size_t smem, cudaStream_t st);
@@ -142,9 +143,9 @@ cudaError_t launch_spectral_receivers(const DevSiRow* rows, int n_rows, const fl
 cudaError_t launch_server_receivers(const DevSrvReceiver* rec, int n_rec, const DevDomain* doms, const float* set,
                                     float* aux, int* scene_step, const int* scene_limit, const int* slots, int n_slots,
                                     cudaStream_t st, const int* counts = nullptr);
-// dense p0 = px + py of the given domains into dst (frames); sub > 1 keeps
 // dense p0 = px + py of one domain
 cudaError_t launch_field_sum(const float* px, const float* py, int pitch, int rows, int cols, float* dst, cudaStream_t st);
+// dense p0 = px + py of the given domains into dst (frames); sub > 1 keeps
 // every sub-th row and column (ceil(nx/sub) x ceil(ny/sub) values per domain);
 // n_rec floats of rec_src (a receiver row) are copied to rec_dst on the way
 cudaError_t launch_frame(const int* doms_idx, const long long* dst_off, int n, const DevDomain* doms, const float* set,

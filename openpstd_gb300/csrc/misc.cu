@@ -28,9 +28,17 @@ const StageVariant* stage_variants_tma_b(int L, int* n);
 
 const StageVariant* stage_variants_quad_a(int L, int* n);
 const StageVariant* stage_variants_quad_b(int L, int* n);
+const StageVariant* stage_variants_quad_c(int L, int* n);
+const StageVariant* stage_variants_quad_d(int L, int* n);
 
-static const StageVariant* stage_variants_quad(int L, int* n) {
-    return L <= 512 ? stage_variants_quad_a(L, n) : stage_variants_quad_b(L, n);
+static std::vector<StageVariant> stage_variants_quad(int L) {
+    std::vector<StageVariant> out;
+    int n = 0;
+    const StageVariant* v = L <= 512 ? stage_variants_quad_a(L, &n) : stage_variants_quad_b(L, &n);
+    out.insert(out.end(), v, v + n);
+    v = L <= 512 ? stage_variants_quad_c(L, &n) : stage_variants_quad_d(L, &n);   // fused forms
+    out.insert(out.end(), v, v + n);
+    return out;
 }
 
 static const StageVariant* stage_variants_tma(int L, int* n) {
@@ -66,8 +74,8 @@ int stage_variants(int L, const StageVariant** out) {
             else v = stage_variants_huge(len, &n);
             for (int i = 0; i < nf; i++) all[lg].push_back(f[i]);
             for (int i = 0; i < nt; i++) all[lg].push_back(tv[i]);
-            int nd = 0, nq = 0, i = 0;
-            const StageVariant* qv = stage_variants_quad(len, &nq);
+            const std::vector<StageVariant> qv = stage_variants_quad(len);
+            int nd = 0, nq = (int)qv.size(), i = 0;
             while (i < n && !v[i].bf16) all[lg].push_back(v[i++]);
             if (i < n) {   // the precision-study variants come last in their lists
                 for (int q = 0; q < nq; q++) all[lg].push_back(qv[q]);
@@ -271,14 +279,6 @@ __global__ void frame_kernel(const int* idx, const long long* dst_off, int n, co
         }
 }
 
-cudaError_t launch_pml_post(const int* idx, int n, int blocks, const DevDomain* doms, float* set, float* fixed,
-                            float* p0, const float* att, cudaStream_t st, const int* off) {
-    if (n <= 0 || blocks <= 0) return cudaSuccess;
-    const dim3 grid = off ? dim3(blocks, 1) : dim3(blocks, n);
-    pml_post_kernel<<<grid, 128, 0, st>>>(idx, n, off, doms, set, fixed, p0, att);
-    return cudaGetLastError();
-}
-
 // dense p0 = px + py of one domain (snapshots)
 __global__ void field_sum_kernel(const float* __restrict__ px, const float* __restrict__ py, int pitch, int rows, int cols,
                                  float* __restrict__ dst) {
@@ -291,6 +291,14 @@ __global__ void field_sum_kernel(const float* __restrict__ px, const float* __re
 
 cudaError_t launch_field_sum(const float* px, const float* py, int pitch, int rows, int cols, float* dst, cudaStream_t st) {
     field_sum_kernel<<<std::min(rows, 2048), 256, 0, st>>>(px, py, pitch, rows, cols, dst);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_pml_post(const int* idx, int n, int blocks, const DevDomain* doms, float* set, float* fixed,
+                            float* p0, const float* att, cudaStream_t st, const int* off) {
+    if (n <= 0 || blocks <= 0) return cudaSuccess;
+    const dim3 grid = off ? dim3(blocks, 1) : dim3(blocks, n);
+    pml_post_kernel<<<grid, 128, 0, st>>>(idx, n, off, doms, set, fixed, p0, att);
     return cudaGetLastError();
 }
 

@@ -22,7 +22,7 @@ __device__ __forceinline__ void pml_post_block(int dj, int lb, const int* idx, c
     const int r = lb / chunks, i = ((lb - r * chunks) << 7) + threadIdx.x;
     if (r < d.ny && i < d.nx) {
         const long long e = (long long)r * d.pitch_p + i;
-        const float px = base[d.o_px + e], py = base[d.o_py + e];
+        const float px = __ldcg(base + d.o_px + e), py = __ldcg(base + d.o_py + e);
         p0[d.o_p0 + e] = __fadd_rn(px, py);
         if (d.att_xp >= 0) base[d.o_px + e] = __fmul_rn(px, att[d.att_xp + i]);
         if (d.att_yp >= 0) base[d.o_py + e] = __fmul_rn(py, att[d.att_yp + r]);
@@ -30,11 +30,11 @@ __device__ __forceinline__ void pml_post_block(int dj, int lb, const int* idx, c
     if (d.fixed) {
         if (r < d.ny && i < d.nx + 1 && d.att_xv >= 0) {
             const long long e = d.o_vx + (long long)r * d.pitch_vx + i;
-            base[e] = __fmul_rn(base[e], att[d.att_xv + i]);
+            base[e] = __fmul_rn(__ldcg(base + e), att[d.att_xv + i]);
         }
         if (r < d.ny + 1 && i < d.nx && d.att_yv >= 0) {
             const long long e = d.o_vy + (long long)r * d.pitch_vy + i;
-            base[e] = __fmul_rn(base[e], att[d.att_yv + r]);
+            base[e] = __fmul_rn(__ldcg(base + e), att[d.att_yv + r]);
         }
     }
 }

@@ -195,6 +195,8 @@ struct Server {
     DevBuf<int> scene_limit;                   // steps requested per slot
     DevBuf<DevSrvReceiver> drec;
     DevBuf<int> dslots;
+    DevBuf<int> init_words;                    // speakers and domain origins of newly admitted scenes
+    DevBuf<float> frame_buf;                   // final frames on their way out
     std::vector<float> att;
     std::map<std::tuple<int, int, int, float, float, float>, int> att_off;
     std::map<int64_t, std::unique_ptr<Request>> reqs;
@@ -549,16 +551,22 @@ struct Server {
             base.push_back(total);
             total += c;
         }
-        DevBuf<DevJob> nb;
-        nb.alloc(std::max<size_t>(total, 1));
-        CK(cudaMemsetAsync(nb.p, 0, nb.n * sizeof(DevJob), K.stream));
-        for (size_t r = 0; r < regs.size(); r++)
-            if (regs[r].a.cap)
-                CK(cudaMemcpyAsync(nb.p + base[r], K.djobs_all.p + regs[r].base, regs[r].a.cap * sizeof(DevJob),
-                                   cudaMemcpyDeviceToDevice, K.stream));
-        CK(cudaStreamSynchronize(K.stream));   // before the old array is freed
-        std::swap(K.djobs_all.p, nb.p);
-        std::swap(K.djobs_all.n, nb.n);
+        // set 0 keeps plan entries, set 1 the four-strip form's records
+        auto move = [&](auto& buf) {
+            using T = std::remove_reference_t<decltype(*buf.p)>;
+            std::remove_reference_t<decltype(buf)> nb;
+            nb.alloc(std::max<size_t>(total, 1));
+            CK(cudaMemsetAsync(nb.p, 0, nb.n * sizeof(T), K.stream));
+            for (size_t r = 0; r < regs.size(); r++)
+                if (regs[r].a.cap)
+                    CK(cudaMemcpyAsync(nb.p + base[r], buf.p + regs[r].base, regs[r].a.cap * sizeof(T),
+                                       cudaMemcpyDeviceToDevice, K.stream));
+            CK(cudaStreamSynchronize(K.stream));   // before the old array is freed
+            std::swap(buf.p, nb.p);
+            std::swap(buf.n, nb.n);
+        };
+        if (pset == 0) move(K.djobs_all);
+        else move(K.dqjobs_all);
         for (size_t r = 0; r < regs.size(); r++) {
             regs[r].base = base[r];
             regs[r].a.grow(caps[r]);
@@ -620,6 +628,13 @@ struct Server {
         for (const auto& kv : q->jobs) {   // (the array has its final layout now)
             const auto [r, off] = q->job_ranges[i++];
             if (kv.second.empty()) continue;
+            if (pset == 1) {
+                std::vector<QJob> g = Kernel::quad_jobs_of(kv.second, hd);
+                for (QJob& j : g) j.dom += o;
+                CK(cudaMemcpyAsync(K.dqjobs_all.p + regs[r].base + off, g.data(), g.size() * sizeof(QJob),
+                                   cudaMemcpyHostToDevice, K.stream));
+                continue;
+            }
             std::vector<DevJob> g = kv.second;
             for (DevJob& j : g) {
                 j.dom += o;
@@ -639,7 +654,10 @@ struct Server {
         for (const auto& kv : q->jobs) {
             const auto [r, off] = q->job_ranges[i++];
             if (kv.second.empty()) continue;
-            CK(cudaMemsetAsync(K.djobs_all.p + regs[r].base + off, 0, kv.second.size() * sizeof(DevJob), K.stream));
+            if (pset == 0)
+                CK(cudaMemsetAsync(K.djobs_all.p + regs[r].base + off, 0, kv.second.size() * sizeof(DevJob), K.stream));
+            else
+                CK(cudaMemsetAsync(K.dqjobs_all.p + regs[r].base + off, 0, kv.second.size() * sizeof(QJob), K.stream));
             regs[r].a.release(off, kv.second.size());
         }
         adom.release(q->dom_off, q->local.size());
@@ -657,6 +675,7 @@ struct Server {
             K.ddoms.alloc(adom.cap);
             regs.clear();
             K.djobs_all.alloc(1);
+            K.dqjobs_all.alloc(1);
             if (pset == 0) {
                 regs.resize(2);
                 regs[0].L = 1024;
@@ -666,7 +685,7 @@ struct Server {
                 CK(prepare_stage_all(K.merged_fam));
             }
             for (Request* q : active) q->placed = false;
-            if (K.counters.n < 6 * MAX_REGIONS) K.counters.alloc(6 * MAX_REGIONS);
+            if (K.counters.n < 6) K.counters.alloc(6);
             filt_up = tw_up = win_up = 0;
             moved = true;
         }
@@ -735,21 +754,36 @@ struct Server {
             CK(cudaMemcpyAsync(scene_limit.p + q->slot, &q->n_steps, sizeof(int), cudaMemcpyHostToDevice, K.stream));
             static const int one = 1;
             CK(cudaMemcpyAsync(K.first_step.p + q->slot, &one, sizeof(int), cudaMemcpyHostToDevice, K.stream));
-            const Scene& sc = q->scene;
-            if (!sc.speakers.empty()) {
-                std::vector<int> x0, y0;
-                for (auto& d : sc.doms) { x0.push_back(d.x0); y0.push_back(d.y0); }
-                std::vector<DevSpeaker> spk;
-                for (auto& s : sc.speakers) spk.push_back({s.x, s.y});
-                DevBuf<int> dx0, dy0;
-                DevBuf<DevSpeaker> dspk;
-                dx0.upload(x0);
-                dy0.upload(y0);
-                dspk.upload(spk);
-                CK(launch_speakers(K.ddoms.p + q->dom_off, dx0.p, dy0.p, (int)sc.doms.size(), dspk.p, (int)spk.size(),
-                                   sc.s.dx, sc.s.band_width, K.sets[K.cur].p, K.fixed.p, K.p0.p, K.stream));
-                CK(cudaStreamSynchronize(K.stream));
+        }
+        // the speakers and domain origins of all of them in one upload (the
+        // buffer is kept: an allocation and its release per scene cost more
+        // than the scene's steps)
+        std::vector<int> words;
+        for (Request* q : fresh) {
+            for (auto& d : q->scene.doms) words.push_back(d.x0);
+            for (auto& d : q->scene.doms) words.push_back(d.y0);
+            for (auto& s : q->scene.speakers) {
+                int w[2];
+                const DevSpeaker v{s.x, s.y};
+                static_assert(sizeof v == sizeof w, "two words per speaker");
+                std::memcpy(w, &v, sizeof w);
+                words.push_back(w[0]);
+                words.push_back(w[1]);
             }
+        }
+        if (!words.empty()) {
+            if (init_words.n < words.size()) init_words.alloc(2 * words.size());
+            CK(cudaMemcpyAsync(init_words.p, words.data(), words.size() * sizeof(int), cudaMemcpyHostToDevice, K.stream));
+        }
+        size_t at = 0;
+        for (Request* q : fresh) {
+            const Scene& sc = q->scene;
+            const int nd = (int)sc.doms.size(), ns = (int)sc.speakers.size();
+            const int* x0 = init_words.p + at;
+            if (ns)
+                CK(launch_speakers(K.ddoms.p + q->dom_off, x0, x0 + nd, nd, reinterpret_cast<const DevSpeaker*>(x0 + 2 * nd),
+                                   ns, sc.s.dx, sc.s.band_width, K.sets[K.cur].p, K.fixed.p, K.p0.p, K.stream));
+            at += 2 * nd + 2 * ns;
         }
         CK(cudaStreamSynchronize(K.stream));
     }
@@ -758,22 +792,43 @@ struct Server {
     // state set of its last step
     void final_frame(Request* q) {
         q->frame.assign(q->frame_f, 0.f);
-        size_t at = 0;
-        std::vector<float> a, b;
+        // summed on the device, one copy (blocks of at most 64 MiB of whole rows)
+        size_t cap = std::min<size_t>((size_t)q->frame_f, 16 << 20), row = 1;
+        for (const DevDomain& d : q->local) row = std::max(row, (size_t)d.nx);
+        if (frame_buf.n < cap) {   // smaller blocks where device memory is short
+            frame_buf.release();
+            while (cudaMalloc(&frame_buf.p, cap * sizeof(float)) != cudaSuccess) {
+                cudaGetLastError();
+                frame_buf.p = nullptr;
+                if (cap <= row) throw CudaError("no device memory for a row of a final frame");
+                cap = std::max(row, cap / 4);
+            }
+            frame_buf.n = cap;
+        }
+        size_t at = 0, held = 0;
+        auto flush = [&]() {
+            if (held) CK(cudaMemcpyAsync(q->frame.data() + at, frame_buf.p, held * sizeof(float), cudaMemcpyDeviceToHost, K.stream));
+            CK(cudaStreamSynchronize(K.stream));
+            at += held;
+            held = 0;
+        };
         for (size_t k = 0; k < q->local.size(); k++) {
             const DevDomain& d = q->local[k];
             if (d.pml) continue;
             const float* base = d.fixed ? K.fixed.p + q->fixed_off : K.sets[q->final_set].p + q->set_off;
-            const size_t n = (size_t)d.nx * d.ny;
-            a.resize(n);
-            b.resize(n);
-            CK(cudaMemcpy2D(a.data(), d.nx * sizeof(float), base + d.o_px, d.pitch_p * sizeof(float), d.nx * sizeof(float),
-                            d.ny, cudaMemcpyDeviceToHost));
-            CK(cudaMemcpy2D(b.data(), d.nx * sizeof(float), base + d.o_py, d.pitch_p * sizeof(float), d.nx * sizeof(float),
-                            d.ny, cudaMemcpyDeviceToHost));
-            for (size_t i = 0; i < n; i++) q->frame[at + i] = a[i] + b[i];
-            at += n;
+            for (int r = 0; r < d.ny;) {
+                const int nr = (int)std::min<size_t>(d.ny - r, (frame_buf.n - held) / d.nx);
+                if (nr == 0) {
+                    flush();
+                    continue;
+                }
+                const long long e = (long long)r * d.pitch_p;
+                CK(launch_field_sum(base + d.o_px + e, base + d.o_py + e, d.pitch_p, nr, d.nx, frame_buf.p + held, K.stream));
+                held += (size_t)nr * d.nx;
+                r += nr;
+            }
         }
+        flush();
     }
 
     // info[4] = {active, queued, finished in this tick, steps advanced}.  The

@@ -9,10 +9,14 @@
 // are resident (with job record and tables read) when the previous stage ends,
 // and a step is seven nodes in a row instead of fifteen with forks.
 //
-// Two families: 0 has small jobs of 128 threads and tables in shared memory
-// (many SMs, short passes: scenes that do not fill the GPU); 1 has 256 threads
-// and more strips per job.  The plan times both on the scene's own steps against
-// the per-length launches and keeps the fastest.
+// Three families: 0 has small jobs of 128 threads and tables in shared memory
+// (many SMs: scenes that do not fill the GPU); 1 has 256 threads and more
+// strips per job; 2 has family 0's jobs with 256 threads and smaller radices,
+// because in a small scene a stage lasts as long as its last CTA and a CTA as
+// long as one thread's passes.  Step of the 200 x 200 scene: per-length launches
+// 61 us, family 0 55, 1 66, 2 49; of a 611 x 405 scene in six domains: 93, 89,
+// 86, 109.  The plan times them on the scene's own steps against the per-length
+// launches and keeps the fastest.
 #include "pml_post.cuh"
 #include "stage_quad.cuh"
 
@@ -41,6 +45,21 @@ struct ChainFam1 {
     using C2048 = QCfg<2048, 1, 256, 3, 4, 8, 8, 8>;
     using C4096 = QCfg<4096, 1, 256, 3, 8, 8, 8, 8>;
     using C8192 = QCfg<8192, 1, 256, 3, 16, 8, 8, 8>;
+};
+
+// family 0's job sizes with twice the threads and smaller radices: shorter
+// passes for the last CTA of a stage
+struct ChainFam2 {
+    static constexpr int NT = 256, MINB = 2;
+    using C32 = QCfg<32, 8, 256, 2, 4, 8, 0, 0, 1>;
+    using C64 = QCfg<64, 8, 256, 2, 4, 4, 4, 0, 1>;
+    using C128 = QCfg<128, 8, 256, 2, 4, 4, 8, 0, 1>;
+    using C256 = QCfg<256, 4, 256, 2, 4, 4, 4, 4, 1>;
+    using C512 = QCfg<512, 2, 256, 2, 4, 4, 4, 8, 1>;
+    using C1024 = QCfg<1024, 1, 256, 2, 4, 4, 8, 8, 1>;
+    using C2048 = QCfg<2048, 1, 256, 2, 4, 8, 8, 8, 1>;
+    using C4096 = QCfg<4096, 1, 256, 2, 8, 8, 8, 8, 1>;
+    using C8192 = QCfg<8192, 1, 256, 2, 16, 8, 8, 8, 0>;
 };
 
 // (not inlined: every length keeps its own register allocation)
@@ -89,14 +108,16 @@ static const StageVariant* chain_variants(int L) {
 }
 
 const StageVariant* chain_variant(int L, int fam) {
-    return fam == 1 ? chain_variants<ChainFam1>(L) : chain_variants<ChainFam0>(L);
+    return fam == 2 ? chain_variants<ChainFam2>(L) : fam == 1 ? chain_variants<ChainFam1>(L) : chain_variants<ChainFam0>(L);
 }
 
 template <class F>
 static cudaError_t prepare_fam() {
     return cudaFuncSetAttribute(stage_chain<F>, cudaFuncAttributeMaxDynamicSharedMemorySize, F::C8192::SMEM);
 }
-cudaError_t prepare_chain(int fam) { return fam == 1 ? prepare_fam<ChainFam1>() : prepare_fam<ChainFam0>(); }
+cudaError_t prepare_chain(int fam) {
+    return fam == 2 ? prepare_fam<ChainFam2>() : fam == 1 ? prepare_fam<ChainFam1>() : prepare_fam<ChainFam0>();
+}
 
 // launch `kernel` so that it may start while its predecessor in the stream drains
 template <class... P, class... Q>
@@ -111,13 +132,20 @@ static cudaError_t launch_pdl(void (*kernel)(P...), int grid, int threads, size_
     cfg.stream = st;
     cfg.attrs = &at;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, std::forward<Q>(args)...);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args...);
+    if (e == cudaErrorNotSupported || e == cudaErrorInvalidValue) {   // a stream without the attribute: plain order
+        cudaGetLastError();
+        cfg.numAttrs = 0;
+        e = cudaLaunchKernelEx(&cfg, kernel, args...);
+    }
+    return e;
 }
 
 cudaError_t launch_chain(int fam, int n_jobs, const StageArgs& a, size_t smem, cudaStream_t st) {
     if (n_jobs <= 0) return cudaSuccess;
-    return fam == 1 ? launch_pdl(stage_chain<ChainFam1>, n_jobs, ChainFam1::NT, smem, st, a)
-                    : launch_pdl(stage_chain<ChainFam0>, n_jobs, ChainFam0::NT, smem, st, a);
+    return fam == 2   ? launch_pdl(stage_chain<ChainFam2>, n_jobs, ChainFam2::NT, smem, st, a)
+           : fam == 1 ? launch_pdl(stage_chain<ChainFam1>, n_jobs, ChainFam1::NT, smem, st, a)
+                      : launch_pdl(stage_chain<ChainFam0>, n_jobs, ChainFam0::NT, smem, st, a);
 }
 
 // After the sixth stage: blocks below `pml_blocks` do the PML multiply

@@ -1,8 +1,9 @@
 // stage_quad.cuh -- one RK stage with four real strips per transform unit.
 //
-// A quad is four adjacent strips of one job: two complex strips A = s0 + i s2
-// and B = s1 + i s3, stored position by position as one 16-byte element
-// (s0, s1, s2, s3) = (re A, re B, im A, im B).  What this buys over the
+// A quad is four adjacent strips of one job: two complex strips A = s0 + i s1
+// and B = s2 + i s3 (neighbours share a transform, and with it its rounding:
+// their amplitudes are closest), stored position by position as one 16-byte
+// element (s0, s2, s1, s3) = (re A, re B, im A, im B).  What this buys over the
 // complex-strip form of stage_kernel.cuh, which computes the same transform
 // with the same constants:
 //   * a column job's element is four adjacent columns of one row, i.e. one
@@ -21,6 +22,12 @@
 // data -- two dependent round trips where the plain form chains five (job,
 // domain, first-step flag, neighbour domain, data).  That chain, not the
 // arithmetic, is what a stage of a small scene spends its time on.
+//
+// Measured (GB300, one RK stage of a 96-scene batch, complex-strip form -> this
+// one, us): length 128 237 -> 169, 256 107 -> 73, 512 159 -> 117, 1024 174 ->
+// 139, 2048 52 -> 49; length 8192 of the 8192^2 scene 2822 -> 2360.  What bounds
+// it there: the L1 data path (66-75 % of its wavefronts; DRAM 27-35 %, issue
+// 36-44 %, ncu), i.e. the passes' trips through shared memory.
 //
 // The kernels may be launched with programmatic stream serialisation: a CTA
 // reads its record and copies its tables before it waits for the previous
@@ -165,9 +172,10 @@ struct QDFT<16, INV> {
 // L, quads per CTA, threads, min CTAs per SM, radices; TSM = 1: twiddles and
 // the job's filter are copied to shared memory while the strips are on their
 // way (a CTA that runs alone on its SM finds them in no cache)
-template <int L_, int CS_, int NT_, int MINB_, int R0_, int R1_, int R2_ = 0, int R3_ = 0, int TSM_ = 0>
+// FUSE = 1: the last pass updates the fields itself
+template <int L_, int CS_, int NT_, int MINB_, int R0_, int R1_, int R2_ = 0, int R3_ = 0, int TSM_ = 0, int FUSE_ = 0>
 struct QCfg {
-    static constexpr int L = L_, CS = CS_, NT = NT_, MINB = MINB_, TSM = TSM_, CTW = 1;
+    static constexpr int L = L_, CS = CS_, NT = NT_, MINB = MINB_, TSM = TSM_, CTW = 1, FUSE = FUSE_;
     static constexpr int R0 = R0_, R1 = R1_, R2 = R2_, R3 = R3_;
     static constexpr int NP = R3_ ? 4 : (R2_ ? 3 : 2);
     static_assert(R0 * R1 * (R2 ? R2 : 1) * (R3 ? R3 : 1) == L, "radix plan must multiply to L");
@@ -184,8 +192,16 @@ struct QCfg {
     static constexpr int T2 = T1 + (NP > 2 ? (M1 / R1) * tw_entry(R1) : 0);
     static constexpr int TWN = T2 + (NP > 3 ? (M2 / R2) * tw_entry(R2) : 0);
     static constexpr int DATA = CS * SP * 16;
-    static constexpr int SMEM = DATA + (TSM ? (TWN + L) * 8 : 0);
+    static constexpr int JOB = DATA + (TSM ? (TWN + L) * 8 : 0);   // byte offset of the job record's copy
+    static constexpr int SMEM = JOB + (int)sizeof(QJob);
+    static_assert(sizeof(QJob) % 16 == 0 && JOB % 16 == 0, "the record is copied in 16-byte pieces");
     static constexpr int TPQ = NT / CS;   // threads per quad in gather and epilogue
+    // 16-byte loads of a column job's thread in flight (two fields each), and
+    // row-job chunks: twice as many where a thread has that many elements and
+    // the register budget is 100 and more (shorter strips: the loads past the
+    // end cost a small scene's chained step 10 us of 55)
+    static constexpr int UC = 65536 / (NT * MINB) >= 100 && L / TPQ >= 16 ? 8 : 4;
+    static constexpr int PRE = UC == 8;   // stage-start values loaded ahead of the last inverse pass
 };
 
 template <class C>
@@ -255,8 +271,9 @@ __device__ __forceinline__ void qmid_pass(float4* sm, const float4* filt, int ti
     }
 }
 
+// all passes but the last inverse one
 template <class C>
-__device__ __forceinline__ void qconvolve(float4* sm, const float2* tw, const float4* filt, int tid, int z0, int lo, int hi) {
+__device__ __forceinline__ void qconvolve(float4* sm, const float2* tw, const float4* filt, int tid, int z0) {
     qfwd_pass<C, C::R0, C::L, 0, true>(sm, tw, tid, z0);
     __syncthreads();
     if constexpr (C::NP > 2) {
@@ -277,8 +294,6 @@ __device__ __forceinline__ void qconvolve(float4* sm, const float2* tw, const fl
         qinv_pass<C, C::R1, C::M1, C::T1, false>(sm, tw, tid, 0, 0);
         __syncthreads();
     }
-    qinv_pass<C, C::R0, C::L, 0, true>(sm, tw, tid, lo, hi);
-    __syncthreads();
 }
 
 // ---------------------------------------------------------------- loads
@@ -347,119 +362,161 @@ __device__ __forceinline__ float4 qband(float4 raw, float4 mir, float T, float R
 // Strips to positions W .. W+n of each quad, the two interface bands around
 // them.  The neighbours' values are loaded before the strips, the mirrored own
 // values are read back from shared memory (the strip's ends), so every field
-// value is loaded once.
-template <class C, bool YDIR, bool TWO>
-__device__ __forceinline__ void qstrips(float4* smq, const QPtr& own, const QJob& J, int g, int l) {
-    const int n = J.n, W = J.W, count = J.count;
-    if constexpr (YDIR) {
-        if (own.flags & QS_ALIGNED) {
-            const float* a = own.a + 4 * g;
-            const float* b = TWO ? own.b + 4 * g : nullptr;
-            const bool part = 4 * g + 4 > count;
-#pragma unroll 1
-            for (int i0 = l; i0 < n; i0 += 4 * C::TPQ) {
-                float4 u[4];
+// value is loaded once.  All loads of a thread are issued before the first one
+// is used (sums px + py come after them): with a sum behind every load a job
+// paid one memory round trip per load.
+__device__ __forceinline__ float4 qperm(float4 v) { return make_float4(v.x, v.z, v.y, v.w); }   // strips <-> element
+
+enum QKind { QK_ROWS, QK_COLS, QK_ANY };   // x strips; y strips on 16-byte boundaries; y strips elsewhere
+
+__device__ __forceinline__ float4 qmask(float4 v, int m) {   // keep the first m strips
+    if (m < 1) v.x = 0.f;
+    if (m < 2) v.y = 0.f;
+    if (m < 3) v.z = 0.f;
+    if (m < 4) v.w = 0.f;
+    return v;
+}
+
+template <class C, int KIND, bool TWO>
+__device__ __forceinline__ void qgather_k(float4* smq, const StageArgs& A, const QJob& J, const QPtr& own, const QPtr& lo,
+                                          const QPtr& hi, int g, int l) {
+    constexpr int TPQ = C::TPQ, NB = (64 + TPQ - 1) / TPQ < 4 ? (64 + TPQ - 1) / TPQ : 4;
+    const bool vel = J.kind & JK_VEL, h1 = !(lo.flags & QS_NONE), h2 = !(hi.flags & QS_NONE);
+    const int W = J.W, n = J.n, s0 = 4 * g, m = J.count - s0;   // m: live strips of the quad
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    const float* wl = A.win + J.wtab;   // window.head(W) at 0, its tail at W + 1
+    float4 ra[NB], rb[NB];
+    float wv[NB];
 #pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    const int i = i0 + q * C::TPQ;
-                    if (i < n && 4 * g < count) {
-                        u[q] = qld4(a + (long long)i * own.pitch);
-                        if (TWO) u[q] = add4(u[q], qld4(b + (long long)i * own.pitch));
-                    } else {
-                        u[q] = make_float4(0.f, 0.f, 0.f, 0.f);
-                    }
-                    if (part) {
-                        if (4 * g + 2 > count) u[q].y = 0.f;
-                        if (4 * g + 3 > count) u[q].z = 0.f;
-                        u[q].w = 0.f;
-                    }
-                }
-#pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    const int i = i0 + q * C::TPQ;
-                    if (i < n) smq[qoff<C>(W + i)] = u[q];
-                }
+    for (int q = 0; q < NB; q++) {
+        const int j = l + q * TPQ;
+        const bool low = j < W, need = j < 2 * W && m > 0 && (low ? h1 : h2);
+        const float *sa = low ? lo.a : hi.a, *sb = low ? lo.b : hi.b;
+        const long long pitch = low ? lo.pitch : hi.pitch;
+        const int pos = low ? j : j - W;
+        ra[q] = rb[q] = zero;
+        wv[q] = 0.f;
+        if (j < 2 * W) wv[q] = __ldg(wl + j + (low ? 0 : 1));
+        if constexpr (KIND == QK_ROWS) {
+            const float *pa = sa + s0 * pitch + pos, *pb = sb + s0 * pitch + pos;
+            if (need) ra[q].x = qld(pa);
+            if (need && m > 1) ra[q].y = qld(pa + pitch);
+            if (need && m > 2) ra[q].z = qld(pa + 2 * pitch);
+            if (need && m > 3) ra[q].w = qld(pa + 3 * pitch);
+            if constexpr (TWO) {
+                const bool nb = need && sb;
+                if (nb) rb[q].x = qld(pb);
+                if (nb && m > 1) rb[q].y = qld(pb + pitch);
+                if (nb && m > 2) rb[q].z = qld(pb + 2 * pitch);
+                if (nb && m > 3) rb[q].w = qld(pb + 3 * pitch);
             }
+        } else if constexpr (KIND == QK_COLS) {
+            const long long e = pos * pitch + s0;
+            if (need) ra[q] = qld4(sa + e);
+            if (TWO && need && sb) rb[q] = qld4(sb + e);
         } else {
-            for (int i = l; i < n; i += C::TPQ) smq[qoff<C>(W + i)] = qelem(own, true, g, i, count);
-        }
-    } else {
-        // four rows, four positions each: rows start on 128-byte boundaries and
-        // are padded past their last quad
-        const int chunks = (n + 3) >> 2, s0 = 4 * g;
-        const float* a = own.a + (long long)s0 * own.pitch;
-        const float* b = TWO ? own.b + (long long)s0 * own.pitch : nullptr;
-#pragma unroll 1
-        for (int c = l; c < chunks; c += C::TPQ) {
-            const int i = c << 2;
-            float4 u[4];
-#pragma unroll
-            for (int r = 0; r < 4; r++) {
-                u[r] = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (s0 + r < count) {
-                    u[r] = qld4(a + (long long)r * own.pitch + i);
-                    if (TWO) u[r] = add4(u[r], qld4(b + (long long)r * own.pitch + i));
-                }
-            }
-            const int p = W + i;
-            smq[qoff<C>(p)] = make_float4(u[0].x, u[1].x, u[2].x, u[3].x);
-            if (i + 1 < n) smq[qoff<C>(p + 1)] = make_float4(u[0].y, u[1].y, u[2].y, u[3].y);
-            if (i + 2 < n) smq[qoff<C>(p + 2)] = make_float4(u[0].z, u[1].z, u[2].z, u[3].z);
-            if (i + 3 < n) smq[qoff<C>(p + 3)] = make_float4(u[0].w, u[1].w, u[2].w, u[3].w);
+            if (need) ra[q] = qelem(low ? lo : hi, true, g, pos, J.count);
         }
     }
+    if constexpr (KIND == QK_COLS) {
+        const float *a = own.a + s0, *b = own.b + s0;
+        const long long pitch = own.pitch;
+#pragma unroll 1
+        for (int i0 = l; i0 < n; i0 += C::UC * TPQ) {
+            float4 ua[C::UC], ub[C::UC];
+#pragma unroll
+            for (int q = 0; q < C::UC; q++) {
+                const int i = i0 + q * TPQ;
+                ua[q] = ub[q] = zero;
+                if (i < n && m > 0) ua[q] = qld4(a + i * pitch);
+                if (TWO && i < n && m > 0 && own.b) ub[q] = qld4(b + i * pitch);
+            }
+#pragma unroll
+            for (int q = 0; q < C::UC; q++) {
+                const int i = i0 + q * TPQ;
+                if constexpr (TWO) ua[q] = add4(ua[q], ub[q]);
+                if (m < 4) ua[q] = qmask(ua[q], m);
+                if (i < n) smq[qoff<C>(W + i)] = qperm(ua[q]);
+            }
+        }
+    } else if constexpr (KIND == QK_ROWS) {
+        // four rows, four positions each: rows start on 128-byte boundaries and
+        // are padded past their last quad
+        const int chunks = (n + 3) >> 2;
+        const long long pitch = own.pitch;
+        const float *a = own.a + s0 * pitch, *b = own.b + s0 * pitch;
+        constexpr int UR = C::UC / 4;
+#pragma unroll 1
+        for (int c0 = l; c0 < chunks; c0 += UR * TPQ) {
+            float4 u[UR][4], v[UR][4];
+#pragma unroll
+            for (int h = 0; h < UR; h++) {
+                const int i = (c0 + h * TPQ) << 2;
+#pragma unroll
+                for (int r = 0; r < 4; r++) {
+                    u[h][r] = v[h][r] = zero;
+                    if (r < m && i < n) u[h][r] = qld4(a + r * pitch + i);
+                    if (TWO && r < m && i < n && own.b) v[h][r] = qld4(b + r * pitch + i);
+                }
+            }
+#pragma unroll
+            for (int h = 0; h < UR; h++) {
+                const int i = (c0 + h * TPQ) << 2, p = W + i;
+                if constexpr (TWO) {
+#pragma unroll
+                    for (int r = 0; r < 4; r++) u[h][r] = add4(u[h][r], v[h][r]);
+                }
+                if (i < n) smq[qoff<C>(p)] = make_float4(u[h][0].x, u[h][2].x, u[h][1].x, u[h][3].x);
+                if (i + 1 < n) smq[qoff<C>(p + 1)] = make_float4(u[h][0].y, u[h][2].y, u[h][1].y, u[h][3].y);
+                if (i + 2 < n) smq[qoff<C>(p + 2)] = make_float4(u[h][0].z, u[h][2].z, u[h][1].z, u[h][3].z);
+                if (i + 3 < n) smq[qoff<C>(p + 3)] = make_float4(u[h][0].w, u[h][2].w, u[h][1].w, u[h][3].w);
+            }
+        }
+    } else {
+#pragma unroll 1
+        for (int i = l; i < n; i += TPQ) smq[qoff<C>(W + i)] = m > 0 ? qperm(qelem(own, true, g, i, J.count)) : zero;
+    }
+    __syncthreads();
+    auto store = [&](int j, float4 r, float w) {
+        const bool low = j < W;
+        const int mp = low ? (vel ? W - j : W - 1 - j) : (vel ? n - 2 - (j - W) : n - 1 - (j - W));   // mirrored own position
+        const float4 v = qband(qperm(r), smq[qoff<C>(W + mp)], low ? J.T1 : J.T2, low ? J.R1 : J.R2, w);
+        smq[qoff<C>(low ? j : n + j)] = (low ? h1 : h2) ? v : zero;
+    };
+#pragma unroll
+    for (int q = 0; q < NB; q++) {
+        const int j = l + q * TPQ;
+        if constexpr (TWO && KIND != QK_ANY) ra[q] = add4(ra[q], rb[q]);
+        if (KIND == QK_COLS && m < 4) ra[q] = qmask(ra[q], m);
+        if (j < 2 * W) store(j, ra[q], wv[q]);
+    }
+#pragma unroll 1
+    for (int j = l + NB * TPQ; j < 2 * W; j += TPQ) {   // windows wider than 32
+        const bool low = j < W;
+        const float4 r = m > 0 && (low ? h1 : h2) ? qelem(low ? lo : hi, KIND != QK_ROWS, g, low ? j : j - W, J.count) : zero;
+        store(j, r, __ldg(wl + j + (low ? 0 : 1)));
+    }
+    __syncthreads();
 }
 
 template <class C>
 __device__ __forceinline__ void qgather(float4* sm, const StageArgs& A, const QJob& J, int tid) {
     const bool vel = J.kind & JK_VEL, ydir = J.kind & JK_Y;
-    const bool first = A.stage == 0 && A.first_step[J.scene] != 0;
+    const bool first = A.stage == 0 && __ldcg(A.first_step + J.scene) != 0;
     // column jobs: neighbouring threads on neighbouring quads of one row; row
     // jobs: on neighbouring positions of one quad
     const int g = ydir ? tid % C::CS : tid / C::TPQ, l = ydir ? tid / C::CS : tid % C::TPQ;
     float4* smq = sm + g * C::SP;
-    const QPtr own = qsource(A, J.own, vel, first);
-    const QPtr lo = qsource(A, J.lo, vel, first), hi = qsource(A, J.hi, vel, first);
-    const bool h1 = !(lo.flags & QS_NONE), h2 = !(hi.flags & QS_NONE);
-    const int W = J.W, n = J.n, count = J.count;
-    constexpr int NB = (64 + C::TPQ - 1) / C::TPQ < 4 ? (64 + C::TPQ - 1) / C::TPQ : 4;
-    float4 raw[NB];
-    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-    auto load = [&](int j) {
-        if (j < W) return h1 ? qelem(lo, ydir, g, j, count) : zero;
-        return h2 ? qelem(hi, ydir, g, j - W, count) : zero;
-    };
-#pragma unroll
-    for (int q = 0; q < NB; q++) {
-        const int j = l + q * C::TPQ;
-        raw[q] = (j < 2 * W && 4 * g < count) ? load(j) : zero;
-    }
-    if (ydir) {
-        if (own.b) qstrips<C, true, true>(smq, own, J, g, l);
-        else qstrips<C, true, false>(smq, own, J, g, l);
+    const QPtr own = qsource(A, J.own, vel, first), lo = qsource(A, J.lo, vel, first), hi = qsource(A, J.hi, vel, first);
+    if (!ydir) {
+        if (vel) qgather_k<C, QK_ROWS, false>(smq, A, J, own, lo, hi, g, l);
+        else qgather_k<C, QK_ROWS, true>(smq, A, J, own, lo, hi, g, l);
+    } else if ((own.flags & QS_ALIGNED) && (lo.flags & (QS_ALIGNED | QS_NONE)) && (hi.flags & (QS_ALIGNED | QS_NONE))) {
+        if (vel) qgather_k<C, QK_COLS, false>(smq, A, J, own, lo, hi, g, l);
+        else qgather_k<C, QK_COLS, true>(smq, A, J, own, lo, hi, g, l);
     } else {
-        if (own.b) qstrips<C, false, true>(smq, own, J, g, l);
-        else qstrips<C, false, false>(smq, own, J, g, l);
+        qgather_k<C, QK_ANY, true>(smq, A, J, own, lo, hi, g, l);
     }
-    __syncthreads();
-    const float* wl = A.win + J.wtab;   // window.head(W); its tail starts at W + 1
-    auto store = [&](int j, float4 r) {
-        if (j < W) {
-            const int m = vel ? W - j : W - 1 - j;
-            smq[qoff<C>(j)] = h1 ? qband(r, smq[qoff<C>(W + m)], J.T1, J.R1, __ldg(wl + j)) : zero;
-        } else {
-            const int jj = j - W, m = vel ? n - 2 - jj : n - 1 - jj;
-            smq[qoff<C>(W + n + jj)] = h2 ? qband(r, smq[qoff<C>(W + m)], J.T2, J.R2, __ldg(wl + W + 1 + jj)) : zero;
-        }
-    };
-#pragma unroll
-    for (int q = 0; q < NB; q++) {
-        const int j = l + q * C::TPQ;
-        if (j < 2 * W) store(j, raw[q]);
-    }
-#pragma unroll 1
-    for (int j = l + NB * C::TPQ; j < 2 * W; j += C::TPQ) store(j, 4 * g < count ? load(j) : zero);
-    __syncthreads();
 }
 
 // ---------------------------------------------------------------- epilogue
@@ -474,8 +531,37 @@ __device__ __forceinline__ float2 qrk(float2 p, float2 d, float cdt, float rho, 
     }
 }
 
+// Stage-start values of a thread's first outputs, loaded before the last
+// inverse pass (where the register budget allows): that pass hides their latency.
+template <class C>
+struct QPrev {
+    float4 v[C::UC];
+};
+template <class C>
+__device__ __forceinline__ void qprefetch(QPrev<C>& P, const StageArgs& A, const QJob& J, int tid) {
+    const bool ydir = J.kind & JK_Y;
+    const int g = ydir ? tid % C::CS : tid / C::TPQ, l = ydir ? tid / C::CS : tid % C::TPQ;
+    const int count = J.count, nout = (J.kind & JK_VEL) ? J.n - 1 : J.n + 1, s0 = 4 * g;
+    const long long pitch = J.pitch_out;
+    const float* prev = A.prev + J.o_out;
+    if (ydir) {
+        if (!(J.own.flags & QS_ALIGNED) || s0 + 4 > count) return;
+#pragma unroll
+        for (int q = 0; q < C::UC; q++) {
+            const int i = l + q * C::TPQ;
+            if (i < nout) P.v[q] = qld4(prev + i * pitch + s0);
+        }
+    } else {
+#pragma unroll
+        for (int q = 0; q < C::UC; q++) {
+            const int i = (l + (q >> 2) * C::TPQ) << 2, r = q & 3;
+            if (i < nout && s0 + r < count) P.v[q] = qld4(prev + (s0 + r) * pitch + i);
+        }
+    }
+}
+
 template <class C, bool VEL, bool ATT, bool YDIR>
-__device__ __forceinline__ void qepilogue_k(const float4* sm, const StageArgs& A, const QJob& J, int tid) {
+__device__ __forceinline__ void qepilogue_k(const float4* sm, const StageArgs& A, const QJob& J, int tid, const QPrev<C>& P) {
     const int g = YDIR ? tid % C::CS : tid / C::TPQ, l = YDIR ? tid / C::CS : tid % C::TPQ;
     const float4* smq = sm + g * C::SP;
     const int W = J.W, count = J.count, nout = VEL ? J.n - 1 : J.n + 1, s0 = 4 * g;
@@ -488,18 +574,19 @@ __device__ __forceinline__ void qepilogue_k(const float4* sm, const StageArgs& A
     if constexpr (YDIR) {
         if ((J.own.flags & QS_ALIGNED) && s0 + 4 <= count) {
 #pragma unroll 1
-            for (int i0 = l; i0 < nout; i0 += 4 * C::TPQ) {
-                float4 pv[4];
+            for (int i0 = l; i0 < nout; i0 += C::UC * C::TPQ) {
+                float4 pv[C::UC];
 #pragma unroll
-                for (int q = 0; q < 4; q++) {
+                for (int q = 0; q < C::UC; q++) {
                     const int i = i0 + q * C::TPQ;
-                    if (i < nout) pv[q] = qld4(prev + i * pitch + s0);
+                    if (C::PRE && i0 == l) pv[q] = P.v[q];
+                    else if (i < nout) pv[q] = qld4(prev + i * pitch + s0);
                 }
 #pragma unroll
-                for (int q = 0; q < 4; q++) {
+                for (int q = 0; q < C::UC; q++) {
                     const int i = i0 + q * C::TPQ;
                     if (i >= nout) break;
-                    const float4 d = smq[qoff<C>(W + i)];
+                    const float4 d = qperm(smq[qoff<C>(W + i)]);
                     float2 u = qrk<VEL>(make_float2(pv[q].x, pv[q].y), make_float2(d.x, d.y), cdt, rho, c2, rinv);
                     float2 v = qrk<VEL>(make_float2(pv[q].z, pv[q].w), make_float2(d.z, d.w), cdt, rho, c2, rinv);
                     if constexpr (ATT) {
@@ -513,7 +600,7 @@ __device__ __forceinline__ void qepilogue_k(const float4* sm, const StageArgs& A
         } else {
 #pragma unroll 1
             for (int i = l; i < nout; i += C::TPQ) {
-                const float4 d4 = smq[qoff<C>(W + i)];
+                const float4 d4 = qperm(smq[qoff<C>(W + i)]);
                 const float d[4] = {d4.x, d4.y, d4.z, d4.w};
 #pragma unroll
                 for (int q = 0; q < 4; q++) {
@@ -532,7 +619,10 @@ __device__ __forceinline__ void qepilogue_k(const float4* sm, const StageArgs& A
             float4 pv[4];
 #pragma unroll
             for (int r = 0; r < 4; r++)
-                if (s0 + r < count) pv[r] = qld4(prev + (s0 + r) * pitch + i);   // rows are padded past their last quad
+                if (C::PRE && c == l) pv[r] = P.v[r];
+                else if (C::PRE && C::UC == 8 && c == l + C::TPQ) pv[r] = P.v[r + C::UC - 4];
+                else if (s0 + r < count) pv[r] = qld4(prev + (s0 + r) * pitch + i);   // rows are padded past their last quad
+                else pv[r] = make_float4(0.f, 0.f, 0.f, 0.f);
             float4 d[4];
 #pragma unroll
             for (int e = 0; e < 4; e++) d[e] = i + e < nout ? smq[qoff<C>(W + i + e)] : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -547,7 +637,7 @@ __device__ __forceinline__ void qepilogue_k(const float4* sm, const StageArgs& A
                 float v[4] = {pv[r].x, pv[r].y, pv[r].z, pv[r].w};
 #pragma unroll
                 for (int e = 0; e < 4; e++) {
-                    const float dv = r == 0 ? d[e].x : r == 1 ? d[e].y : r == 2 ? d[e].z : d[e].w;
+                    const float dv = r == 0 ? d[e].x : r == 1 ? d[e].z : r == 2 ? d[e].y : d[e].w;
                     v[e] = rk_update(v[e], dv, VEL, cdt, rho, c2, rinv);
                     if constexpr (ATT) v[e] = __fmul_rn(v[e], a[e]);
                 }
@@ -565,50 +655,164 @@ __device__ __forceinline__ void qepilogue_k(const float4* sm, const StageArgs& A
 }
 
 template <class C>
-__device__ __forceinline__ void qepilogue(const float4* sm, const StageArgs& A, const QJob& J, int tid) {
+__device__ __forceinline__ void qepilogue(const float4* sm, const StageArgs& A, const QJob& J, int tid, const QPrev<C>& P) {
     const bool ydir = J.kind & JK_Y;
     if (J.kind & JK_VEL) {
-        if (ydir) qepilogue_k<C, true, false, true>(sm, A, J, tid);
-        else qepilogue_k<C, true, false, false>(sm, A, J, tid);
+        if (ydir) qepilogue_k<C, true, false, true>(sm, A, J, tid, P);
+        else qepilogue_k<C, true, false, false>(sm, A, J, tid, P);
     } else if (A.last && J.att >= 0) {   // PML multiply of vx / vy at the sixth stage
-        if (ydir) qepilogue_k<C, false, true, true>(sm, A, J, tid);
-        else qepilogue_k<C, false, true, false>(sm, A, J, tid);
+        if (ydir) qepilogue_k<C, false, true, true>(sm, A, J, tid, P);
+        else qepilogue_k<C, false, true, false>(sm, A, J, tid, P);
     } else {
-        if (ydir) qepilogue_k<C, false, false, true>(sm, A, J, tid);
-        else qepilogue_k<C, false, false, false>(sm, A, J, tid);
+        if (ydir) qepilogue_k<C, false, false, true>(sm, A, J, tid, P);
+        else qepilogue_k<C, false, false, false>(sm, A, J, tid, P);
     }
+}
+
+// ---------------------------------------------------------------- fused last pass
+// A thread of the last inverse pass updates the elements it ends up with: saves
+// the trip of the results through shared memory and a barrier, but reaches row
+// jobs' fields with 4-byte accesses.  The same for the first pass (each thread
+// loading its own elements, mirrored values read twice) was 1.1-1.9 times
+// slower at every length and is not here.
+
+// m: live strips of the quad (1..4)
+template <bool VEC>
+__device__ __forceinline__ float4 qfetch(const float* p, long long ss, int m) {
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (!p) return v;
+    if constexpr (VEC) {
+        v = qld4(p);
+    } else {
+        v.x = qld(p);
+        if (m > 1) v.y = qld(p + ss);
+        if (m > 2) v.z = qld(p + 2 * ss);
+        if (m > 3) v.w = qld(p + 3 * ss);
+    }
+    return v;
+}
+
+template <class C, bool VEL, bool ATT, bool VEC>
+__device__ __forceinline__ void qlast_pass(float4* sm, const StageArgs& A, const QJob& J, const float2* tw, int tid) {
+    constexpr int R = C::R0, Q = C::L / R, ITEMS = C::CS * Q;
+    const bool ydir = J.kind & JK_Y;
+    const int W = J.W, count = J.count, nout = VEL ? J.n - 1 : J.n + 1;
+    const float cdt = J.cdt[A.stage], rho = J.rho, c2 = J.c2, rinv = J.rinv;
+    const long long sp = ydir ? J.pitch_out : 1, ss = ydir ? 1 : J.pitch_out;
+#pragma unroll 1
+    for (int it = tid; it < ITEMS; it += C::NT) {
+        const int g = ydir ? it % C::CS : it / Q, n1 = ydir ? it / C::CS : it % Q;
+        const int m = count - 4 * g;
+        if (m <= 0) continue;
+        const float4* base = sm + g * C::SP + n1 + (n1 >> C::SH);
+        float2 w[R];
+        pass_twiddles<C, R, C::TSM != 0>(tw, n1, w);
+        Q2 x[R];
+        x[0] = q_of(base[0]);
+#pragma unroll
+        for (int k = 1; k < R; k++) x[k] = qmulc(q_of(base[qoff<C>(k * Q)]), w[k]);
+        QDFT<R, true>::run(x);
+        const long long o = J.o_out + (long long)(4 * g) * ss + (n1 - W) * sp;   // output of q: + q * Q * sp
+        const float* prev = A.prev + o;
+        float* out = A.out + o;
+        const float* att = A.att + J.att + n1 - W;
+        constexpr int G = R < 4 ? R : 4;
+#pragma unroll
+        for (int q0 = 0; q0 < R; q0 += G) {
+            float4 pv[G];
+#pragma unroll
+            for (int u = 0; u < G; u++) {
+                const int i = n1 + (q0 + u) * Q - W;
+                pv[u] = qfetch<VEC>(i >= 0 && i < nout ? prev + (q0 + u) * Q * sp : nullptr, ss, m);
+            }
+#pragma unroll
+            for (int u = 0; u < G; u++) {
+                const int q = q0 + u, i = n1 + q * Q - W;
+                if (i < 0 || i >= nout) continue;
+                float2 a = qrk<VEL>(make_float2(pv[u].x, pv[u].z), x[q].re, cdt, rho, c2, rinv);
+                float2 b = qrk<VEL>(make_float2(pv[u].y, pv[u].w), x[q].im, cdt, rho, c2, rinv);
+                if constexpr (ATT) {
+                    const float t = __ldg(att + q * Q);
+                    a = mul2(a, make_float2(t, t));
+                    b = mul2(b, make_float2(t, t));
+                }
+                float* d = out + q * Q * sp;
+                if (VEC && m >= 4) {
+                    *reinterpret_cast<float4*>(d) = make_float4(a.x, b.x, a.y, b.y);
+                } else {
+                    d[0] = a.x;
+                    if (m > 1) d[ss] = b.x;
+                    if (m > 2) d[2 * ss] = a.y;
+                    if (m > 3) d[3 * ss] = b.y;
+                }
+            }
+        }
+    }
+}
+
+template <class C, bool VEC>
+__device__ __forceinline__ void qlast(float4* sm, const StageArgs& A, const QJob& J, const float2* tw, int tid) {
+    if (J.kind & JK_VEL) qlast_pass<C, true, false, VEC>(sm, A, J, tw, tid);
+    else if (A.last && J.att >= 0) qlast_pass<C, false, true, VEC>(sm, A, J, tw, tid);
+    else qlast_pass<C, false, false, VEC>(sm, A, J, tw, tid);
 }
 
 // ---------------------------------------------------------------- kernels
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
-// one job: tables (TSM) before the previous launch is waited for
+// strips, transform, update of one job
 template <class C>
-__device__ __forceinline__ void quad_job(float4* sm, const StageArgs& A, const QJob& J, const float2* tw_global, int tid) {
+__device__ __forceinline__ void quad_body(float4* sm, const StageArgs& A, const QJob& J, const float2* tw, const float4* filt,
+                                          int tid) {
+    qgather<C>(sm, A, J, tid);
+    const int lo = J.W, hi = J.W + ((J.kind & JK_VEL) ? J.n - 1 : J.n + 1);
+    qconvolve<C>(sm, tw, filt, tid, 2 * J.W + J.n);
+    QPrev<C> P;
+    if constexpr (!C::FUSE) {
+        if constexpr (C::PRE) qprefetch<C>(P, A, J, tid);
+        qinv_pass<C, C::R0, C::L, 0, true>(sm, tw, tid, lo, hi);
+        __syncthreads();
+    }
+    if constexpr (C::FUSE) {
+        if ((J.kind & JK_Y) && (J.own.flags & QS_ALIGNED)) qlast<C, true>(sm, A, J, tw, tid);
+        else qlast<C, false>(sm, A, J, tw, tid);
+    } else {
+        qepilogue<C>(sm, A, J, tid, P);
+    }
+}
+
+// one job: its record (and, TSM, tables) into shared memory before the
+// previous launch is waited for -- read where it is used, its second line cost
+// a job of a small scene another memory round trip
+template <class C>
+__device__ __forceinline__ void quad_job(float4* sm, const StageArgs& A, const QJob& job, const float2* tw_global, int tid) {
     const float2* tw = tw_global;
-    const float4* filt = reinterpret_cast<const float4*>(A.filt + J.dtab);
+    const float4* filt = reinterpret_cast<const float4*>(A.filt + job.dtab);
+    auto copy = [&](float4* d, const float4* s) {
+        const unsigned a = (unsigned)__cvta_generic_to_shared(d);
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(a), "l"(s) : "memory");
+    };
+    float4* js = sm + C::JOB / 16;
+    if (tid < (int)sizeof(QJob) / 16) copy(js + tid, reinterpret_cast<const float4*>(&job) + tid);
+    asm volatile("cp.async.commit_group;" ::: "memory");
     if constexpr (C::TSM) {
         float4* tws = sm + C::DATA / 16;
         float4* fls = tws + C::TWN / 2;
         const float4* t4 = reinterpret_cast<const float4*>(tw_global);
-        auto copy = [&](float4* d, const float4* s) {
-            const unsigned a = (unsigned)__cvta_generic_to_shared(d);
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(a), "l"(s) : "memory");
-        };
         for (int i = tid; i < C::TWN / 2; i += C::NT) copy(tws + i, t4 + i);
         for (int i = tid; i < C::L / 2; i += C::NT) copy(fls + i, filt + i);
-        asm volatile("cp.async.commit_group;" ::: "memory");
         tw = reinterpret_cast<const float2*>(tws);
         filt = fls;
     }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    asm volatile("cp.async.wait_group 1;" ::: "memory");   // the record
+    __syncthreads();
+    const QJob& J = *reinterpret_cast<const QJob*>(js);
     grid_wait();
     grid_release();
-    if constexpr (C::TSM) asm volatile("cp.async.wait_all;" ::: "memory");   // made visible by the gather's barriers
-    qgather<C>(sm, A, J, tid);
-    const bool vel = J.kind & JK_VEL;
-    qconvolve<C>(sm, tw, filt, tid, 2 * J.W + J.n, J.W, J.W + (vel ? J.n - 1 : J.n + 1));
-    qepilogue<C>(sm, A, J, tid);
+    asm volatile("cp.async.wait_group 0;" ::: "memory");   // the tables: visible after the gather's barriers
+    quad_body<C>(sm, A, J, tw, filt, tid);
 }
 
 template <class C>
@@ -622,6 +826,48 @@ __global__ void __launch_bounds__(C::NT, C::MINB) stage_quad(const __grid_consta
         return;
     }
     quad_job<C>(smq, A, J, A.tw, threadIdx.x);
+}
+
+// Serving loop: resident CTAs walk a record table whose length is read from
+// device memory, with a stride of the grid (records of one launch have one
+// length, so a job counter -- an atomic round trip and a barrier per job --
+// would balance little).  Free entries (all zero) and jobs of scenes that have
+// taken all their steps are skipped.
+template <class C>
+__global__ void __launch_bounds__(C::NT, C::MINB) stage_quad_dev(const __grid_constant__ StageArgs A, const int* count) {
+    extern __shared__ __align__(16) float4 smq[];
+    static_assert(!C::TSM, "the serving loop reads its tables through L1");
+    const int n = *count;
+    for (int j = blockIdx.x; j < n; j += gridDim.x) {
+        const QJob& J = A.qjobs[j];
+        const bool copy = J.kind & JK_COPY;
+        if ((J.L == 0 && !copy) || (A.scene_limit && A.scene_step[J.scene] >= A.scene_limit[J.scene])) continue;
+        if (copy) {
+            copy_axis<C::NT>(A, A.doms[J.dom], J.kind & JK_Y, threadIdx.x);
+            continue;
+        }
+        quad_body<C>(smq, A, J, A.tw, reinterpret_cast<const float4*>(A.filt + J.dtab), threadIdx.x);
+        __syncthreads();   // shared memory is the next job's
+    }
+}
+
+template <class C>
+cudaError_t launch_quad_dev_t(const int* count, const StageArgs& a, cudaStream_t st) {
+    static int grid = 0;
+    if (grid == 0) {
+        int dev, sms, per = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, stage_quad_dev<C>, C::NT, C::SMEM);
+        grid = sms * (per > 0 ? per : 1);
+    }
+    stage_quad_dev<C><<<grid, C::NT, C::SMEM, st>>>(a, count);
+    return cudaGetLastError();
+}
+
+template <class C>
+cudaError_t prepare_quad_dev_t() {
+    return cudaFuncSetAttribute(stage_quad_dev<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
 }
 
 template <class C>
@@ -654,6 +900,15 @@ StageVariant make_quad_variant(const char* name) {
     v.prepare = &prepare_quad_t<C>;
     v.smem_for = &quad_smem<C>;
     v.name = name;
+    return v;
+}
+
+// with the serving loop's form
+template <class C>
+StageVariant make_quad_dev_variant(const char* name) {
+    StageVariant v = make_quad_variant<C>(name);
+    v.launch_dev = &launch_quad_dev_t<C>;
+    v.prepare_dev = &prepare_quad_dev_t<C>;
     return v;
 }
 

@@ -13,6 +13,7 @@ const StageVariant* stage_variants_quad_a(int L, int* n) {
     static const StageVariant v128[] = {
         make_quad_variant<QCfg<128, 8, 128, 6, 8, 16>>("L128 quad8 nt128 r8.16"),
         make_quad_variant<QCfg<128, 8, 128, 7, 4, 4, 8>>("L128 quad8 nt128 r4.4.8"),
+        make_quad_variant<QCfg<128, 8, 128, 6, 4, 4, 8>>("L128 quad8 nt128 mb6 r4.4.8"),
         make_quad_variant<QCfg<128, 8, 64, 10, 16, 8>>("L128 quad8 nt64 r16.8"),
         make_quad_variant<QCfg<128, 16, 128, 5, 16, 8>>("L128 quad16 nt128 r16.8"),
         make_quad_variant<QCfg<128, 4, 64, 14, 4, 4, 8, 0, 1>>("L128 quad4 nt64 r4.4.8 tsm"),
@@ -25,6 +26,7 @@ const StageVariant* stage_variants_quad_a(int L, int* n) {
     };
     static const StageVariant v512[] = {
         make_quad_variant<QCfg<512, 2, 128, 7, 8, 8, 8>>("L512 quad2 nt128 r8.8.8"),
+        make_quad_variant<QCfg<512, 2, 128, 6, 8, 8, 8>>("L512 quad2 nt128 mb6 r8.8.8"),
         make_quad_variant<QCfg<512, 4, 256, 3, 8, 8, 8>>("L512 quad4 nt256 r8.8.8"),
         make_quad_variant<QCfg<512, 1, 64, 14, 8, 8, 8>>("L512 quad1 nt64 r8.8.8"),
         make_quad_variant<QCfg<512, 2, 128, 6, 8, 8, 8, 0, 1>>("L512 quad2 nt128 r8.8.8 tsm"),
@@ -33,9 +35,9 @@ const StageVariant* stage_variants_quad_a(int L, int* n) {
     switch (L) {
         case 32: *n = 1; return v32;
         case 64: *n = 1; return v64;
-        case 128: *n = 5; return v128;
+        case 128: *n = 6; return v128;
         case 256: *n = 4; return v256;
-        case 512: *n = 5; return v512;
+        case 512: *n = 6; return v512;
         default: *n = 0; return nullptr;
     }
 }

@@ -7,11 +7,15 @@ const StageVariant* stage_variants_quad_b(int L, int* n) {
     static const StageVariant v1024[] = {
         make_quad_variant<QCfg<1024, 1, 128, 7, 8, 16, 8>>("L1024 quad1 nt128 r8.16.8"),
         make_quad_variant<QCfg<1024, 2, 128, 4, 16, 8, 8>>("L1024 quad2 nt128 r16.8.8"),
+        make_quad_variant<QCfg<1024, 1, 64, 8, 16, 8, 8>>("L1024 quad1 nt64 r16.8.8"),
+        make_quad_variant<QCfg<1024, 2, 128, 5, 16, 8, 8>>("L1024 quad2 nt128 mb5 r16.8.8"),
         make_quad_variant<QCfg<1024, 2, 256, 3, 8, 8, 4, 4>>("L1024 quad2 nt256 r8.8.4.4"),
         make_quad_variant<QCfg<1024, 1, 128, 7, 4, 4, 8, 8, 1>>("L1024 quad1 nt128 r4.4.8.8 tsm"),
     };
     static const StageVariant v2048[] = {
         make_quad_variant<QCfg<2048, 1, 128, 4, 16, 16, 8>>("L2048 quad1 nt128 r16.16.8"),
+        make_quad_variant<QCfg<2048, 1, 128, 5, 16, 16, 8>>("L2048 quad1 nt128 mb5 r16.16.8"),
+        make_quad_variant<QCfg<2048, 1, 256, 2, 8, 16, 16>>("L2048 quad1 nt256 r8.16.16"),
         make_quad_variant<QCfg<2048, 1, 256, 3, 4, 8, 8, 8>>("L2048 quad1 nt256 r4.8.8.8"),
         make_quad_variant<QCfg<2048, 2, 256, 2, 16, 16, 8>>("L2048 quad2 nt256 r16.16.8"),
         make_quad_variant<QCfg<2048, 1, 256, 3, 4, 8, 8, 8, 1>>("L2048 quad1 nt256 r4.8.8.8 tsm"),
@@ -26,8 +30,8 @@ const StageVariant* stage_variants_quad_b(int L, int* n) {
         make_quad_variant<QCfg<8192, 1, 1024, 1, 16, 8, 8, 8>>("L8192 quad1 nt1024 r16.8.8.8"),
     };
     switch (L) {
-        case 1024: *n = 4; return v1024;
-        case 2048: *n = 4; return v2048;
+        case 1024: *n = 6; return v1024;
+        case 2048: *n = 6; return v2048;
         case 4096: *n = 3; return v4096;
         case 8192: *n = 2; return v8192;
         default: *n = 0; return nullptr;
