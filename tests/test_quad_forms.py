@@ -94,21 +94,3 @@ def test_chained_receivers_and_steps(oracle_mod, monkeypatch, fam):
     assert np.array_equal(k.receivers(), want)
     assert all(np.array_equal(k.snapshot(i, "px"), p[i]) for i in range(k.domain_count()))
     assert rel(want, np.zeros_like(want)) > 0
-
-
-@pytest.mark.gpu
-@pytest.mark.parametrize("patch", [100.0, 120.0])
-def test_wide_windows(oracle_mod, monkeypatch, patch):
-    """Windows of more than 32 cells (a patch error above 70 dB): more band
-    positions than a thread holds at once."""
-    from openpstd_gb300 import scenes
-    conf = scenes.l_shape(2, scale=0.25, steps=12, pml=70)
-    conf.Settings.SetPatchError(patch)
-    assert 32 < conf.Settings.GetWindowSize() <= 70
-    monkeypatch.setenv("PSTD_CHAIN", "0")
-    check_parity(oracle_mod, conf, 12, threads=16)
-    monkeypatch.delenv("PSTD_CHAIN")
-    monkeypatch.setenv("PSTD_AUTOTUNE", "0")
-    for i in range(3):
-        monkeypatch.setenv("PSTD_PLAN", ",".join(f"{L}:{_quads(L)[i]}" for L in (256, 512)))
-        check_parity(oracle_mod, conf, 12, threads=16)
