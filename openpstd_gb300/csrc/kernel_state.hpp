@@ -509,6 +509,7 @@ struct Kernel {
         q.att = -1;
         q.kind = j.kind;
         q.dom = j.dom;
+        q.scene = doms[j.dom].scene;   // copy jobs too: the serving loop skips jobs by their scene's step count
         q.own.flags = q.lo.flags = q.hi.flags = QS_NONE;
         if (j.kind & JK_COPY) return q;
         const bool vel = j.kind & JK_VEL, y = j.kind & JK_Y;
@@ -518,7 +519,6 @@ struct Kernel {
         q.count = j.count;
         q.n = (y ? d.ny : d.nx) + e;
         q.W = j.W;
-        q.scene = d.scene;
         q.dtab = j.dtab;
         q.wtab = j.wtab;
         q.ttab = j.ttab;

@@ -283,3 +283,27 @@ def test_persistent_tables_grow(monkeypatch, form):
                 assert np.array_equal(rec, want)
             else:
                 assert rel(rec, want) <= 1e-6
+
+
+@pytest.mark.parametrize("form", ["per_length", "merged", "lengths"])
+def test_served_copy_jobs_follow_their_own_scene(monkeypatch, form):
+    """Scenes with PML domains whose x axis is not updated (copy jobs): one
+    that ends first in slot 0, two that go on, and one that joins in the memory
+    the first has left.  Each equals its solo run."""
+    from test_plan_rules import _copying
+    from openpstd_gb300.serving import Server
+    _form_env(monkeypatch, form)
+    cases = [(_copying(lr=("left", "right")), 12), (_copying(lr=(), shift=40), 40),
+             (_copying(lr=("left",), n=(131, 85)), 60), (_copying(lr=("right",)), 30)]
+    with Server(256 << 20, max_scenes=8) as srv:
+        ids = [srv.submit(c, n, final_frame=True) for c, n in cases[:3]]
+        srv.tick(16)
+        assert [srv.poll(i)["state"] for i in ids] == [2, 1, 1]
+        ids.append(srv.submit(*cases[3], final_frame=True))
+        srv.run_until_idle(16)
+        got = [srv.result(i) for i in ids]
+    for i, (c, n) in enumerate(cases):
+        rec, frame = _solo(c, n)
+        assert np.any(rec)
+        assert rel(got[i][0], rec) <= 1e-6, (i, rel(got[i][0], rec))
+        assert rel(got[i][1], frame) <= 1e-6, (i, rel(got[i][1], frame))
