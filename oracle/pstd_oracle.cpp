@@ -94,7 +94,10 @@ static int match_number(int n) { return (int)std::ceil(std::log2((double)n)); }
 
 // kernel/KernelInterface.cpp:128-134
 static int window_size(float patcherror) {
-    int tmp = (int)std::round((patcherror * 0.7 - 17) / 2.);
+    // (volatile: contracted into a fused multiply-subtract, as compilers for Arm
+    // do, 40, 60, 80 and 100 dB round the other way)
+    const volatile double cells = patcherror * 0.7;
+    int tmp = (int)std::round((cells - 17) / 2.);
     tmp = (int)std::round(tmp * 2);
     return tmp;
 }

@@ -41,6 +41,28 @@ def _copying(steps=60, lr=("left",), n=(90, 73), shift=0):
     return conf
 
 
+def test_window_of_every_patch_error(pstd_lib, oracle_mod):
+    """The window is the same in the kernel, the oracle and the Python
+    configuration, whatever machine the library is compiled for."""
+    from openpstd_gb300 import _lib, scenes
+    from openpstd_gb300.config import CConfig, PSTDConfiguration, c_domain_info
+    for patch in range(30, 131):
+        conf = PSTDConfiguration()
+        scenes.base_settings(conf, 4, dx=0.2, pml=101)
+        conf.Settings.SetPatchError(float(patch))
+        conf.Domains = [scenes._domain(0, 0, 411, 411, 0.2, dict(left=0.6, right=0.4, top=0.8, bottom=0.5))]
+        conf.Speakers = conf.Receivers = []
+        cc, h, d = CConfig(conf), ctypes.c_void_p(), c_domain_info()
+        _lib.check(pstd_lib.pstd_scene_build(ctypes.byref(cc.c), ctypes.byref(h)))
+        try:
+            _lib.check(pstd_lib.pstd_scene_domain_info(h, 0, ctypes.byref(d)))
+        finally:
+            pstd_lib.pstd_destroy(h)
+        # kernel/KernelInterface.cpp:128-134 in exact arithmetic: halves round away from zero
+        cells = 2 * ((7 * patch - 170 + 10) // 20)
+        assert d.window[0] == conf.Settings.GetWindowSize() == oracle_mod.window_size(patch) == cells, patch
+
+
 def _records(probe, conf, slot):
     from openpstd_gb300.config import CConfig
     cc = CConfig(conf)
