@@ -161,6 +161,21 @@ inline int planned_variant(int L) {
     return -1;
 }
 
+// The variant of length L that runs untuned and in pstd_solve_noalloc: the
+// first that takes the bucket's windows and needs nothing else of it (one CTA
+// per job over plan entries, no staging row cap or tensor maps, FP32).  Up to
+// 32 cells that is the list's first entry; wider windows get the first plain
+// form.  nullptr: the length is not compiled.
+inline const StageVariant* first_variant(int L, int wmin, int wmax) {
+    const StageVariant* vs;
+    const int nv = stage_variants(L, &vs);
+    for (int i = 0; i < nv; i++) {
+        const StageVariant& v = vs[i];
+        if (!v.persistent && !v.pipe && !v.bf16 && !v.tma && !v.quad && v.fits_window(wmin, wmax)) return &v;
+    }
+    return nullptr;
+}
+
 // Plans chosen by the autotuner, kept per process and keyed by the scene's
 // strip-job structure (like the reference's WisdomCache for FFT plans): a scene
 // tuned once is created again without timing.
@@ -190,6 +205,7 @@ struct Bucket {
     int tw_off = 0;                // float2 offset of the twiddles in dtw
     int fp_off = 0, fv_off = 0;    // float2 offsets of the pressure / velocity filters
     int rc = 4;                    // floats staged per strip by the pipelined form
+    int wmin = 1 << 30, wmax = 0;  // windows of its strips
     bool pinned = false;           // variant fixed by PSTD_PLAN / PSTD_DFT: not tuned
     std::vector<const StageVariant*> cands;   // fastest variants timed alone (refined on whole steps)
     std::string choice;            // autotune record
@@ -439,6 +455,65 @@ struct Kernel {
     static int run_length(const Scene& sc, const StripRun& r) {
         int n = sc.doms[r.dom].len(r.axis);
         return Scene::next_pow2(n + 2 * sc.window_for(n));
+    }
+
+    // the scenes' strips of transform length L: longest strip and windows
+    Bucket bucket_of(int L) const {
+        Bucket b;
+        b.L = L;
+        int longest = 0;
+        for (const Scene& sc : scenes)
+            for (const StripRun& r : sc.runs) {
+                if (run_length(sc, r) != L) continue;
+                const int n = sc.doms[r.dom].len(r.axis), W = sc.window_for(n);
+                longest = std::max(longest, n);
+                b.wmin = std::min(b.wmin, W);
+                b.wmax = std::max(b.wmax, W);
+            }
+        b.rc = (longest + 2 + 3) / 4 * 4;
+        return b;
+    }
+    // the variant can run the bucket's strips: their windows, its staging
+    bool can_run(const StageVariant& v, const Bucket& b) const {
+        return v.fits_window(b.wmin, b.wmax) && v.smem_for(b.rc) <= (size_t)smem_optin;
+    }
+    // ... and the autotuner may choose it (the study forms have other
+    // arithmetic, the staged form needs tensor maps)
+    bool may_tune(const StageVariant& v, const Bucket& b) const {
+        return can_run(v, b) && !v.bf16 && !(v.tma && !dmaps.p);
+    }
+
+    // The variant a bucket starts from: the forced one (index of PSTD_VARIANT,
+    // -1: none) where it can run the strips, else first_variant; PSTD_DFT and
+    // PSTD_PLAN pin one.
+    void choose_variant(Bucket& b, int forced) const {
+        const StageVariant* vs;
+        const int nv = stage_variants(b.L, &vs), nv_fp32 = fp32_variants(vs, nv);
+        b.var = first_variant(b.L, b.wmin, b.wmax);
+        if (!b.var)
+            throw SceneError(PSTD_ERR_UNSUPPORTED, "strip transform length " + std::to_string(b.L) +
+                                                       " is outside the compiled range 32..8192");
+        if (forced >= 0) {
+            const StageVariant* f = &vs[std::min(forced, nv_fp32 - 1)];
+            if (can_run(*f, b)) b.var = f;
+        }
+        if (want_bf16_dft())
+            for (int i = 0; i < nv; i++)
+                if (study_variant_matches(vs[i])) {
+                    b.var = &vs[i];
+                    b.choice = vs[i].tc5 ? " split-TF32 tcgen05 DFT (precision study)"
+                                         : " split-BF16 DFT (precision study)";
+                    b.pinned = true;
+                }
+        if (int i = planned_variant(b.L); i >= 0 && i < nv_fp32) {
+            if (!vs[i].fits_window(b.wmin, b.wmax))
+                throw SceneError(PSTD_ERR_UNSUPPORTED, std::string("PSTD_PLAN: ") + vs[i].name + " does not take windows of " +
+                                                           std::to_string(b.wmin) + " to " + std::to_string(b.wmax) + " cells");
+            b.var = &vs[i];
+            b.choice = " pinned by PSTD_PLAN";
+            b.pinned = true;
+        }
+        if (forced >= 0) b.choice = " pinned";
     }
 
     // all jobs of bucket L for variant v (+ copy jobs if `with_copies`);
@@ -699,36 +774,11 @@ struct Kernel {
             }
         std::sort(Ls.begin(), Ls.end());
         for (int L : Ls) {
+            Bucket b = bucket_of(L);
+            choose_variant(b, forced);
             const StageVariant* vs;
-            int nv = stage_variants(L, &vs);
-            if (nv <= 0)
-                throw SceneError(PSTD_ERR_UNSUPPORTED, "strip transform length " + std::to_string(L) +
-                                                           " is outside the compiled range 32..8192");
+            const int nv = stage_variants(L, &vs);
             for (int i = 0; i < nv; i++) CK(vs[i].prepare());
-            Bucket b;
-            b.L = L;
-            int longest = 0;
-            for (auto& sc : scenes)
-                for (const StripRun& r : sc.runs)
-                    if (run_length(sc, r) == L) longest = std::max(longest, sc.doms[r.dom].len(r.axis));
-            b.rc = (longest + 2 + 3) / 4 * 4;
-            const int nv_fp32 = fp32_variants(vs, nv);
-            b.var = &vs[forced >= 0 ? std::min(forced, nv_fp32 - 1) : 0];
-            if (b.var->smem_for(b.rc) > (size_t)smem_optin) b.var = &vs[0];   // pinned form does not fit
-            if (want_bf16_dft())
-                for (int i = 0; i < nv; i++)
-                    if (study_variant_matches(vs[i])) {
-                        b.var = &vs[i];
-                        b.choice = vs[i].tc5 ? " split-TF32 tcgen05 DFT (precision study)"
-                                             : " split-BF16 DFT (precision study)";
-                        b.pinned = true;
-                    }
-            if (int i = planned_variant(L); i >= 0 && i < nv_fp32) {
-                b.var = &vs[i];
-                b.choice = " pinned by PSTD_PLAN";
-                b.pinned = true;
-            }
-            if (forced >= 0) b.choice = " pinned";
             buckets.push_back(b);
         }
 
@@ -978,14 +1028,12 @@ struct Kernel {
                 std::vector<std::vector<DevJob>> all(nv);
                 std::vector<int> twv(nv), fpv(nv), fvv(nv);
                 for (int i = 0; i < nv; i++) {
+                    if (!may_tune(vs[i], b)) continue;
                     all[i] = make_jobs(b.L, &vs[i], false);
                     twv[i] = twiddles_of(&vs[i]);
                     fpv[i] = filter_of(b.L, false, &vs[i], scenes[0].s.dx);
                     fvv[i] = filter_of(b.L, true, &vs[i], scenes[0].s.dx);
                     if (vs[i].persistent && !one_filter_pair(all[i], fpv[i], fvv[i])) all[i].clear();
-                    if (vs[i].smem_for(b.rc) > (size_t)smem_optin) all[i].clear();   // staging too large
-                    if (vs[i].bf16) all[i].clear();                                  // different arithmetic
-                    if (vs[i].tma && !dmaps.p) all[i].clear();                       // no tensor maps here
                     // length 4096: with strips 0/2 and 1/3 paired, the round-off in a domain the
                     // pulse has not reached was 3.06x the float oracle's (limit 3x) on 4096 x 4096
                     // cells; pinned and served runs only until that is shown to be below it
@@ -993,7 +1041,7 @@ struct Kernel {
                 }
                 upload_tables();
                 float best = 1e30f;
-                int best_i = 0;
+                int best_i = -1;
                 std::string rec;
                 std::vector<std::pair<float, int>> timed;
                 cudaEvent_t e0, e1;
@@ -1034,7 +1082,7 @@ struct Kernel {
                 }
                 cudaEventDestroy(e0);
                 cudaEventDestroy(e1);
-                b.var = &vs[best_i];
+                if (best_i >= 0) b.var = &vs[best_i];
                 b.choice = " tuned" + rec;
                 std::sort(timed.begin(), timed.end());
                 b.cands.clear();
@@ -1051,9 +1099,7 @@ struct Kernel {
             b.fv_off = filter_of(b.L, true, b.var, scenes[0].s.dx);
             if (b.var->persistent && !one_filter_pair(js, b.fp_off, b.fv_off)) {
                 // mixed grid spacings: fall back to the first plain variant
-                const StageVariant* vs;
-                int nv = stage_variants(b.L, &vs);
-                for (int q = 0; q < nv; q++) if (!vs[q].persistent) { b.var = &vs[q]; break; }
+                b.var = first_variant(b.L, b.wmin, b.wmax);
                 js = make_jobs(b.L, b.var, i + 1 == buckets.size());
                 b.tw_off = twiddles_of(b.var);
                 b.choice += " (plain: several grid spacings)";

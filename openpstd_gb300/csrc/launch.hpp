@@ -65,6 +65,11 @@ struct StageVariant {
     bool tc5 = false;                                           // tcgen05 TF32x3 DFT (precision study, opt-in)
     int quad = 0;                                               // four-strip form: jobs are QJob records
     int direct = 0;                                             // direct convolution, Q outputs per task (filter: h)
+    // windows (cells) the form can run: the fused, staged and pipelined forms
+    // keep a strip's interface bands in 32 floats a side, and with a wider
+    // window overwrite the next strip's (past the last strip: other memory)
+    int min_window = 0, max_window = 1 << 30;
+    bool fits_window(int lo, int hi) const { return min_window <= lo && hi <= max_window; }
     cudaError_t (*launch)(int n_jobs, const StageArgs& a, cudaStream_t st);
     cudaError_t (*prepare)();
     size_t (*smem_for)(int row_cap);                            // dynamic shared memory of one CTA

@@ -421,26 +421,21 @@ struct Server {
         for (int L : Ls) {
             const StageVariant* vs;
             const int nv = stage_variants(L, &vs);
-            Bucket b;
-            b.L = L;
-            int longest = 0;
-            for (auto& sc : K.scenes)
-                for (const StripRun& r : sc.runs)
-                    if (Kernel::run_length(sc, r) == L) longest = std::max(longest, sc.doms[r.dom].len(r.axis));
-            b.rc = (longest + 2 + 3) / 4 * 4;
+            Bucket b = K.bucket_of(L);
+            b.var = first_variant(L, b.wmin, b.wmax);
             bool need = false;
             if (forced >= 0) {
-                b.var = &vs[std::min(forced, fp32_variants(vs, nv) - 1)];
+                const StageVariant* f = &vs[std::min(forced, fp32_variants(vs, nv) - 1)];
+                if (K.can_run(*f, b)) b.var = f;
                 b.choice = " pinned";
-            } else if (var_cache.count(L)) {
-                b.var = var_cache[L];
-            } else {
+                CK(b.var->prepare());
+            } else if (var_cache.count(L) && var_cache[L]->fits_window(b.wmin, b.wmax)) {
+                if (K.can_run(*var_cache[L], b)) b.var = var_cache[L];   // else: its staging does not fit
+                CK(b.var->prepare());
+            } else {   // not tuned yet, or for narrower windows
                 for (int i = 0; i < nv; i++) CK(vs[i].prepare());
-                b.var = &vs[0];
                 need = K.autotune;
             }
-            if (b.var->smem_for(b.rc) > (size_t)K.smem_optin) b.var = &vs[0];   // staging of this form does not fit
-            if (forced >= 0) CK(b.var->prepare());
             K.buckets.push_back(b);
             tune.push_back(need);
         }

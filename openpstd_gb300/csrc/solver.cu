@@ -715,11 +715,8 @@ static int solve_noalloc(const pstd_config* config, int n_steps, float* frame_de
     std::vector<DevJob> jobs;
     for (size_t i = 0; i < nbs.size(); i++) {
         NB& b = nbs[i];
-        const StageVariant* vs;
-        const int nv = stage_variants(b.L, &vs);
-        // one CTA per job, no staging row cap, FP32 arithmetic
-        for (int q = 0; q < nv && !b.var; q++)
-            if (!vs[q].persistent && !vs[q].pipe && !vs[q].bf16 && !vs[q].tma && !vs[q].quad) b.var = &vs[q];
+        const Bucket w = kh.bucket_of(b.L);
+        b.var = first_variant(b.L, w.wmin, w.wmax);
         if (!b.var)
             return fail(PSTD_ERR_UNSUPPORTED, "strip transform length " + std::to_string(b.L) +
                                                   " is outside the compiled range 32..8192");

@@ -39,7 +39,7 @@ struct FCfg : Cfg<L_, CS_, NT_, MINB_, R0_, R1_, R2_, R3_> {
     static constexpr int SHF = SHF_;
     static_assert(L_ / R0_ >= 16, "first pass too wide for coalesced row loads");
     // shared memory: the strips, then the blended interface bands of every
-    // real strip (2 x 32 floats: windows are at most 32 wide)
+    // real strip (2 x 32 floats: StageVariant::max_window)
     static constexpr int BAND = 64;
     static constexpr int FSMEM = Cfg<L_, CS_, NT_, MINB_, R0_, R1_, R2_, R3_>::BUF * 8 + 2 * CS_ * BAND * 4;
 };
@@ -502,6 +502,7 @@ StageVariant make_fused_variant(const char* name) {
     v.pipe = false;
     v.bf16 = false;
     v.shf = C::SHF;
+    v.max_window = C::BAND / 2;
     v.launch = &launch_fused_t<C>;
     v.prepare = &prepare_fused_t<C>;
     v.smem_for = &fused_smem<C>;

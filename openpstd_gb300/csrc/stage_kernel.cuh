@@ -1443,7 +1443,7 @@ __global__ void __launch_bounds__(C::NT + C::NTP, 1) stage_ws(StageArgs A, int n
 //   bands[2 sides][2 fields][S2][32]
 // where A = px (or vx, vy, stale p0), B = py (p0 formed as A + B), P = the
 // stage-start values of the updated field.
-constexpr int PIPE_WB = 32;   // band slots per strip (windows are at most 32 wide)
+constexpr int PIPE_WB = 32;   // band slots per strip and side (StageVariant::max_window)
 
 __device__ __forceinline__ void cp16(float* dst, const float* src) {   // both 16-byte aligned
     const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
@@ -1874,6 +1874,7 @@ StageVariant make_pipe_variant(const char* name) {
     v.launch = &launch_pipe_t<C>;
     v.prepare = &prepare_pipe_t<C>;
     v.smem_for = &pipe_smem<C>;
+    v.max_window = PIPE_WB;
     v.name = name;
     return v;
 }

@@ -525,6 +525,7 @@ StageVariant make_tma_variant(const char* name) {
     v.pipe = false;
     v.bf16 = false;
     v.tma = true;
+    v.max_window = 32;   // 64 band floats per strip
     v.ctw = C::CTW;
     v.launch = &launch_tma_t<C>;
     v.prepare = &prepare_tma_t<C>;

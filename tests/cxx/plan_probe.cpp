@@ -39,4 +39,43 @@ int probe_served_records(const pstd_config* cfg, int slot, int* out, int cap) {
     }
 }
 
+// What a scene's plan may run, one line each: "bucket L wmin wmax", then the
+// variant it starts from ("first"), with every PSTD_VARIANT index ("forced i")
+// and those the autotuner may time ("tune"); tensor maps present, staging
+// limit of sm_103a.  PSTD_PLAN and PSTD_DFT are followed.  Returns 0, or the
+// error code with its message in buf.
+int probe_plan(const pstd_config* cfg, char* buf, int cap) {
+    std::string s;
+    int code = 0;
+    Kernel k;
+    static unsigned char map;
+    k.smem_optin = 232448;
+    k.dmaps.p = &map;   // (never read)
+    try {
+        k.build_scenes(cfg, 1);
+        std::map<int, int> lengths;
+        for (const StripRun& r : k.scenes[0].runs) lengths[Kernel::run_length(k.scenes[0], r)]++;
+        for (auto& kv : lengths) {
+            Bucket b = k.bucket_of(kv.first);
+            s += "bucket " + std::to_string(b.L) + " " + std::to_string(b.wmin) + " " + std::to_string(b.wmax) + "\n";
+            k.choose_variant(b, -1);
+            s += std::string("first ") + b.var->name + "\n";
+            const StageVariant* vs;
+            const int nv = stage_variants(b.L, &vs);
+            for (int i = 0; i < nv; i++) {
+                k.choose_variant(b, i);
+                s += "forced " + std::to_string(i) + " " + b.var->name + "\n";
+                if (k.may_tune(vs[i], b)) s += std::string("tune ") + vs[i].name + "\n";
+            }
+        }
+    } catch (SceneError& e) {
+        code = e.code;
+        s = e.what();
+    }
+    k.dmaps.p = nullptr;
+    std::strncpy(buf, s.c_str(), (size_t)cap - 1);
+    buf[cap - 1] = 0;
+    return code;
+}
+
 }  // extern "C"

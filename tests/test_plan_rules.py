@@ -79,3 +79,87 @@ def test_served_records_carry_their_scene(probe, conf):
     r = _records(probe, _copying(**conf), slot=5)
     assert np.any(r[:, 0] & JK_COPY)
     assert np.all(r[:, 1] == 5), r[r[:, 1] != 5]
+
+
+def _plan(probe, conf):
+    """[(L, wmin, wmax, first variant, [variant of PSTD_VARIANT=i], [tuned variants])] of a scene's lengths."""
+    from openpstd_gb300.config import CConfig
+    cc, buf = CConfig(conf), ctypes.create_string_buffer(1 << 17)
+    rc = probe.probe_plan(ctypes.byref(cc.c), buf, len(buf))
+    if rc:
+        return rc, buf.value.decode()
+    out = []
+    for line in buf.value.decode().splitlines():
+        key, rest = line.split(" ", 1)
+        if key == "bucket":
+            out.append([int(v) for v in rest.split()] + [None, [], []])
+        elif key == "first":
+            out[-1][3] = rest
+        elif key == "forced":
+            out[-1][4].append(rest.split(" ", 1)[1])
+        else:
+            out[-1][5].append(rest)
+    return 0, out
+
+
+def _windowed(patch, n=(301, 187), pml=70):
+    """One domain, its strips and those of its PML domains in windows of the patch error's width."""
+    from openpstd_gb300 import scenes
+    from openpstd_gb300.config import PSTDConfiguration
+    conf = PSTDConfiguration()
+    scenes.base_settings(conf, 10, dx=0.2, pml=pml)
+    conf.Settings.SetPatchError(patch)
+    conf.Domains = [scenes._domain(0, 0, *n, 0.2, dict(left=0.6, right=0.4, top=0.8, bottom=0.5))]
+    conf.Speakers = [(n[0] * 0.1, n[1] * 0.1, 0.0)]
+    conf.Receivers = []
+    return conf
+
+
+# the forms that keep a strip's bands in slots of 32 floats a side
+NARROW = (" fused c", " tma", " pipe")
+
+
+def _narrow(name):
+    return any(t in name for t in NARROW) and " quad" not in name
+
+
+@pytest.mark.parametrize("patch,w,pml,n", [(72.0, 34, 40, (41, 50)), (75.0, 36, 50, (301, 187)), (100.0, 54, 70, (301, 187)),
+                                           (100.0, 54, 70, (700, 1200)), (120.0, 68, 70, (2600, 5000))])
+def test_wide_windows_get_no_narrow_form(probe, patch, w, pml, n):
+    """A bucket with a window above 32 cells neither starts from, is forced to
+    nor tunes a form whose band slots hold 32; the other buckets keep theirs."""
+    rc, plan = _plan(probe, _windowed(patch, n, pml))
+    assert rc == 0, plan
+    assert max(b[2] for b in plan) == w
+    for L, wmin, wmax, first, forced, tuned in plan:
+        assert tuned and 0 < wmin <= wmax
+        if wmax > 32:
+            assert not [v for v in [first] + forced + tuned if _narrow(v)], (L, wmax)
+        elif L >= 128:
+            assert _narrow(first) and any(_narrow(v) for v in tuned)
+
+
+def test_windows_up_to_32_start_from_variant_0(probe):
+    import re
+    from openpstd_gb300 import _lib
+    seen = set()
+    for n, pml in [((13, 14), 10), ((21, 25), 20), ((50, 90), 50), ((181, 333), 50), ((611, 1203), 50), ((2003, 4101), 50)]:
+        rc, plan = _plan(probe, _windowed(70.0, n, pml))
+        assert rc == 0, plan
+        for L, _wmin, _wmax, first, forced, tuned in plan:
+            buf, k = ctypes.create_string_buffer(1 << 14), ctypes.c_int32()
+            assert _lib.lib().pstd_stage_variants(L, buf, 1 << 14, ctypes.byref(k)) == 0
+            names = [line.split(" ", 1)[1] for line in buf.value.decode().splitlines()]
+            assert first == names[0] and first in tuned
+            fp32 = [v for v in names if not re.search(r"bf16x3|r16.16.16.2 tcgen05", v)]
+            assert len(forced) == k.value and set(tuned) <= set(fp32)
+            seen.add(L)
+    assert seen == {32, 64, 128, 256, 512, 1024, 2048, 4096, 8192}
+
+
+def test_pinned_plan_refused_where_the_window_is_too_wide(probe, monkeypatch):
+    from openpstd_gb300 import _lib
+    monkeypatch.setenv("PSTD_PLAN", "512:0")
+    assert _plan(probe, _windowed(70.0))[0] == 0
+    rc, msg = _plan(probe, _windowed(100.0))
+    assert rc == _lib.PSTD_ERR_UNSUPPORTED and "does not take windows" in msg
