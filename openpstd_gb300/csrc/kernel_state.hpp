@@ -987,18 +987,21 @@ struct Kernel {
         dmaps.upload(maps);
     }
 
-    // a device error word (a bounded wait that gave up, a job outside a form's
-    // tile) is reported once, here
-    void check_stage_error() {
-        if (!derr.p) return;
+    // the device error word (a bounded wait that gave up, a job outside a
+    // form's tile), cleared
+    int take_stage_error() {
+        if (!derr.p) return 0;
         int e = 0;
         CK(cudaMemcpy(&e, derr.p, sizeof e, cudaMemcpyDeviceToHost));
-        if (e) {
-            CK(cudaMemset(derr.p, 0, sizeof(int)));
+        if (e) CK(cudaMemset(derr.p, 0, sizeof(int)));
+        return e;
+    }
+    // ... reported once, here
+    void check_stage_error() {
+        if (const int e = take_stage_error())
             throw CudaError(e == 3 ? "a stage-kernel job lies outside its form's fixed tile (error 3)"
                                    : "a bounded wait of the stage kernel (TMA copy or tensor-core commit) gave up "
                                      "(error " + std::to_string(e) + ")");
-        }
     }
 
     void upload_tables() {
@@ -1073,6 +1076,10 @@ struct Kernel {
                         float t;
                         CK(cudaEventElapsedTime(&t, e0, e1));
                         ms = std::min(ms, t / reps);
+                    }
+                    if (const int e = take_stage_error()) {   // it skipped work: its time says nothing
+                        rec += " " + std::to_string(i) + ":error " + std::to_string(e);
+                        continue;
                     }
                     char buf[64];
                     std::snprintf(buf, sizeof buf, " %d:%.1fus", i, ms * 1e3f);

@@ -25,8 +25,9 @@
 // wait is bounded: on a timeout the CTA records error 2 in *A.err, waits once
 // more (bounded) for its MMAs, frees its TMEM and leaves.  A job outside the
 // form's fixed tile (window 32, n + 2W <= 128, at most 80 outputs) records
-// error 3 and is not computed; the L = 128 bucket never has one (its strips
-// have n in 32..63 and W = 32).
+// error 3 and is not computed.  L = 128 strips of 32-cell windows always fit
+// (n in 32..63); at other patch errors the length has other windows (26 cells
+// at 60 dB, 36 at 75), so the variants are offered for 32-cell windows only.
 #include "stage_tc5.cuh"
 
 namespace pstd {
@@ -207,6 +208,7 @@ StageVariant make_toe_variant(const char* name) {
     StageVariant v = make_variant<C>(name);
     v.smem = (int)toe_smem<C>();
     v.direct = 8;   // the kernel table of the direct forms (hx, 2L + 8 floats)
+    v.min_window = v.max_window = toe::W;   // the fixed tile
     v.launch = &launch_toe_t<C>;
     v.prepare = &prepare_toe_t<C>;
     v.smem_for = &toe_smem_for<C>;
@@ -505,6 +507,7 @@ StageVariant make_toews_variant(const char* name) {
     StageVariant v = make_variant<C>(name);
     v.smem = (int)toews_smem<C>();
     v.direct = 8;
+    v.min_window = v.max_window = toe::W;
     v.launch = &launch_toews_t<C>;
     v.prepare = &prepare_toews_t<C>;
     v.smem_for = &toews_smem_for<C>;

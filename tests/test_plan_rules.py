@@ -163,3 +163,15 @@ def test_pinned_plan_refused_where_the_window_is_too_wide(probe, monkeypatch):
     assert _plan(probe, _windowed(70.0))[0] == 0
     rc, msg = _plan(probe, _windowed(100.0))
     assert rc == _lib.PSTD_ERR_UNSUPPORTED and "does not take windows" in msg
+
+
+@pytest.mark.parametrize("patch,w,n", [(60.0, 26, (50, 50)), (70.0, 32, (50, 50)), (75.0, 36, (50, 50)), (65.0, 28, (63, 90))])
+def test_toeplitz_forms_for_their_own_window_only(probe, patch, w, n):
+    """The tcgen05 Toeplitz forms compute a fixed tile of 32-cell windows; a
+    bucket of length 128 with other windows is not offered them."""
+    rc, plan = _plan(probe, _windowed(patch, n, pml=50))
+    assert rc == 0, plan
+    L, wmin, wmax, first, forced, tuned = plan[0]
+    assert L == 128 and wmax == w
+    has = [v for v in [first] + forced + tuned if "toeplitz" in v]
+    assert bool(has) == (wmin == wmax == 32), has

@@ -35,7 +35,7 @@ def test_wide_window_parity(oracle_mod, monkeypatch, patch, form):
     k.close()
 
 
-@pytest.mark.parametrize("patch,pml,n", [(100.0, 70, (301, 187)), (100.0, 70, (700, 130))])
+@pytest.mark.parametrize("patch,pml,n", [(75.0, 40, (53, 45)), (100.0, 70, (301, 187)), (100.0, 70, (700, 130))])
 def test_wide_window_every_variant(oracle_mod, monkeypatch, patch, pml, n):
     """Every variant of every length present, pinned: parity, or refused."""
     from openpstd_gb300 import _lib
@@ -104,3 +104,17 @@ def test_wide_windows_served(monkeypatch, form):
     for (rec, frame), conf, n in zip(got, confs, (14, 10)):
         want_rec, want_frame = _solo(conf, n)
         assert rel(rec, want_rec) <= 1e-6 and rel(frame, want_frame) <= 1e-6
+
+
+@pytest.mark.parametrize("form", ["untuned", "tuned", "chain2"])
+@pytest.mark.parametrize("patch,cells", [(60.0, 26), (65.0, 28)])
+def test_narrow_window_parity(oracle_mod, monkeypatch, patch, cells, form):
+    """Windows below 32 cells: length 128 with strips the Toeplitz forms do not take."""
+    from openpstd_gb300 import scenes
+    conf = scenes.l_shape(2, scale=0.25, steps=12)
+    conf.Settings.SetPatchError(patch)
+    assert conf.Settings.GetWindowSize() == cells
+    for k, v in FORMS[form].items():
+        monkeypatch.setenv(k, v)
+    k, _ = check_parity(oracle_mod, conf, 12, threads=16)
+    k.close()
