@@ -867,7 +867,7 @@ struct Kernel {
         if (cacheable) {
             std::lock_guard<std::mutex> lock(plan_cache_mutex());
             auto it = plan_cache().find(sig);
-            if (it != plan_cache().end()) { cached = it->second; hit = true; }
+            if (it != plan_cache().end()) { cached = it->second; hit = plan_applies(cached); }
         }
         reset();
         if (hit) {
@@ -913,6 +913,16 @@ struct Kernel {
         for (auto& b : buckets) choice += " [" + std::string(b.var->name) + b.choice + "]";
         log(PSTD_LOG_DEBUG, std::to_string(scenes.size()) + " scene(s), " + std::to_string(gdom.size()) + " domains, " +
                                 std::to_string(n_rec) + " receivers; stage kernels:" + choice);
+    }
+
+    // every bucket has a variant in the cached plan that can run it
+    bool plan_applies(const PlanChoice& pc) const {
+        for (const Bucket& b : buckets) {
+            bool ok = false;
+            for (const auto& lv : pc.vars) ok |= lv.first == b.L && may_tune(*lv.second, b);
+            if (!ok) return false;
+        }
+        return true;
     }
 
     StageArgs stage_args(int c, int k, const DevJob* jobs, const float2* twp, int fp, int fv, int rc) {
@@ -1325,8 +1335,8 @@ struct Kernel {
     }
 
     // the strip-job structure of the scenes (domain sizes and kinds, every strip
-    // run with its neighbours and transform length): equal signatures get
-    // equal job lists for every variant
+    // run with its neighbours, transform length and window): equal signatures
+    // get equal job lists for every variant, and the same variants can run them
     std::string plan_signature() const {
         std::string s;
         auto put = [&](long long v) { s += std::to_string(v); s += ','; };
@@ -1335,6 +1345,7 @@ struct Kernel {
             for (const Domain& d : sc.doms) { put(d.nx); put(d.ny); put(d.rigid); put(d.pml); put(d.update[0]); put(d.update[1]); }
             for (const StripRun& r : sc.runs) {
                 put(r.dom); put(r.axis); put(r.first); put(r.count); put(r.d1); put(r.d2); put(run_length(sc, r));
+                put(sc.window_for(sc.doms[r.dom].len(r.axis)));
             }
             s += ';';
         }

@@ -78,4 +78,40 @@ int probe_plan(const pstd_config* cfg, char* buf, int cap) {
     return code;
 }
 
+// the plan cache's key of a scene (its length; the text in buf)
+int probe_signature(const pstd_config* cfg, char* buf, int cap) {
+    try {
+        Kernel k;
+        k.build_scenes(cfg, 1);
+        const std::string s = k.plan_signature();
+        std::strncpy(buf, s.c_str(), (size_t)cap - 1);
+        buf[cap - 1] = 0;
+        return (int)s.size();
+    } catch (...) {
+        return -1;
+    }
+}
+
+// 1: the plan that `from` would cache (every length on variant `index`) is
+// accepted for `to`, 0: it is not
+int probe_plan_applies(const pstd_config* from, const pstd_config* to, int index) {
+    Kernel a, b;
+    a.build_scenes(from, 1);
+    b.build_scenes(to, 1);
+    b.smem_optin = 232448;
+    PlanChoice pc;
+    auto lengths = [](Kernel& k) {
+        std::map<int, int> m;
+        for (const StripRun& r : k.scenes[0].runs) m[Kernel::run_length(k.scenes[0], r)]++;
+        return m;
+    };
+    for (auto& kv : lengths(a)) {
+        const StageVariant* vs;
+        stage_variants(kv.first, &vs);
+        pc.vars.push_back({kv.first, &vs[index]});
+    }
+    for (auto& kv : lengths(b)) b.buckets.push_back(b.bucket_of(kv.first));
+    return b.plan_applies(pc);
+}
+
 }  // extern "C"

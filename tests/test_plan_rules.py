@@ -175,3 +175,24 @@ def test_toeplitz_forms_for_their_own_window_only(probe, patch, w, n):
     assert L == 128 and wmax == w
     has = [v for v in [first] + forced + tuned if "toeplitz" in v]
     assert bool(has) == (wmin == wmax == 32), has
+
+
+def test_plan_cache_distinguishes_windows(probe):
+    """Scenes of equal sizes and transform lengths at different patch errors
+    do not share a tuned plan, and one that names a form of too narrow a window
+    is not taken."""
+    from openpstd_gb300.config import CConfig
+    ccs = [CConfig(_windowed(p, (300, 300), pml=50)) for p in (60.0, 70.0, 75.0, 70.2)]
+    sig = []
+    for cc in ccs:
+        buf = ctypes.create_string_buffer(1 << 16)
+        n = probe.probe_signature(ctypes.byref(cc.c), buf, len(buf))
+        assert 0 < n < len(buf)
+        sig.append(buf.value)
+    lengths = [[b[0] for b in _plan(probe, _windowed(p, (300, 300), pml=50))[1]] for p in (60.0, 70.0, 75.0)]
+    assert lengths[0] == lengths[1] == lengths[2] == [128, 512]
+    assert len(set(sig[:3])) == 3
+    assert sig[3] == sig[1]               # 70.2 dB: the same 32 cells
+    at70, at75 = ctypes.byref(ccs[1].c), ctypes.byref(ccs[2].c)
+    assert probe.probe_plan_applies(at70, at70, 0) == 1      # variant 0: the fused form
+    assert probe.probe_plan_applies(at70, at75, 0) == 0
