@@ -478,9 +478,9 @@ struct Kernel {
         return v.fits_window(b.wmin, b.wmax) && v.smem_for(b.rc) <= (size_t)smem_optin;
     }
     // ... and the autotuner may choose it (the study forms have other
-    // arithmetic, the staged form needs tensor maps)
+    // arithmetic, the staged form needs tensor maps, a form may be left out)
     bool may_tune(const StageVariant& v, const Bucket& b) const {
-        return can_run(v, b) && !v.bf16 && !(v.tma && !dmaps.p);
+        return can_run(v, b) && v.tuned && !v.bf16 && !(v.tma && !dmaps.p);
     }
 
     // The variant a bucket starts from: the forced one (index of PSTD_VARIANT,
@@ -1047,10 +1047,6 @@ struct Kernel {
                     fpv[i] = filter_of(b.L, false, &vs[i], scenes[0].s.dx);
                     fvv[i] = filter_of(b.L, true, &vs[i], scenes[0].s.dx);
                     if (vs[i].persistent && !one_filter_pair(all[i], fpv[i], fvv[i])) all[i].clear();
-                    // length 4096: with strips 0/2 and 1/3 paired, the round-off in a domain the
-                    // pulse has not reached was 3.06x the float oracle's (limit 3x) on 4096 x 4096
-                    // cells; pinned and served runs only until that is shown to be below it
-                    if (vs[i].quad && b.L == 4096) all[i].clear();
                 }
                 upload_tables();
                 float best = 1e30f;

@@ -70,6 +70,7 @@ struct StageVariant {
     // window overwrite the next strip's (past the last strip: other memory)
     int min_window = 0, max_window = 1 << 30;
     bool fits_window(int lo, int hi) const { return min_window <= lo && hi <= max_window; }
+    bool tuned = true;                                          // the autotuner may choose it
     cudaError_t (*launch)(int n_jobs, const StageArgs& a, cudaStream_t st);
     cudaError_t (*prepare)();
     size_t (*smem_for)(int row_cap);                            // dynamic shared memory of one CTA

@@ -196,3 +196,15 @@ def test_plan_cache_distinguishes_windows(probe):
     at70, at75 = ctypes.byref(ccs[1].c), ctypes.byref(ccs[2].c)
     assert probe.probe_plan_applies(at70, at70, 0) == 1      # variant 0: the fused form
     assert probe.probe_plan_applies(at70, at75, 0) == 0
+
+
+def test_length_4096_tunes_every_form_within_the_limit(probe):
+    """Every FP32 form of length 4096 may be timed, the four-strip ones (which
+    the chained and served forms run) included, but the one whose round-off
+    was measured above the limit of the large-scene test."""
+    rc, plan = _plan(probe, _windowed(70.0, (2048, 2048), pml=50))
+    assert rc == 0, plan
+    L, _wmin, _wmax, _first, _forced, tuned = plan[-1]
+    assert L == 4096
+    assert "L4096 cs4 nt512 r16.16.16" not in tuned
+    assert sum(" quad" in v for v in tuned) == 5 and sum(" fused c" in v for v in tuned) == 3
