@@ -196,7 +196,6 @@ struct Server {
     DevBuf<DevSrvReceiver> drec;
     DevBuf<int> dslots;
     DevBuf<int> init_words;                    // speakers and domain origins of newly admitted scenes
-    DevBuf<float> frame_buf;                   // final frames on their way out
     std::vector<float> att;
     std::map<std::tuple<int, int, int, float, float, float>, int> att_off;
     std::map<int64_t, std::unique_ptr<Request>> reqs;
@@ -784,46 +783,21 @@ struct Server {
     }
 
     // p0 = px + py of every non-PML domain of a scene, scene order, from the
-    // state set of its last step
+    // state set of its last step: summed on the device into the scene's own
+    // range of another set (which has four fields where the frame has one, and
+    // which nothing reads any more), then one copy -- no device memory of its own
     void final_frame(Request* q) {
         q->frame.assign(q->frame_f, 0.f);
-        // summed on the device, one copy (blocks of at most 64 MiB of whole rows)
-        size_t cap = std::min<size_t>((size_t)q->frame_f, 16 << 20), row = 1;
-        for (const DevDomain& d : q->local) row = std::max(row, (size_t)d.nx);
-        if (frame_buf.n < cap) {   // smaller blocks where device memory is short
-            frame_buf.release();
-            while (cudaMalloc(&frame_buf.p, cap * sizeof(float)) != cudaSuccess) {
-                cudaGetLastError();
-                frame_buf.p = nullptr;
-                if (cap <= row) throw CudaError("no device memory for a row of a final frame");
-                cap = std::max(row, cap / 4);
-            }
-            frame_buf.n = cap;
+        float* dense = K.sets[(q->final_set + 1) % 3].p + q->set_off;
+        size_t at = 0;
+        for (const DevDomain& d : q->local) {
+            if (d.pml) continue;   // (the others are never rigid: their fields lie in the set)
+            const float* base = K.sets[q->final_set].p + q->set_off;
+            CK(launch_field_sum(base + d.o_px, base + d.o_py, d.pitch_p, d.ny, d.nx, dense + at, K.stream));
+            at += (size_t)d.nx * d.ny;
         }
-        size_t at = 0, held = 0;
-        auto flush = [&]() {
-            if (held) CK(cudaMemcpyAsync(q->frame.data() + at, frame_buf.p, held * sizeof(float), cudaMemcpyDeviceToHost, K.stream));
-            CK(cudaStreamSynchronize(K.stream));
-            at += held;
-            held = 0;
-        };
-        for (size_t k = 0; k < q->local.size(); k++) {
-            const DevDomain& d = q->local[k];
-            if (d.pml) continue;
-            const float* base = d.fixed ? K.fixed.p + q->fixed_off : K.sets[q->final_set].p + q->set_off;
-            for (int r = 0; r < d.ny;) {
-                const int nr = (int)std::min<size_t>(d.ny - r, (frame_buf.n - held) / d.nx);
-                if (nr == 0) {
-                    flush();
-                    continue;
-                }
-                const long long e = (long long)r * d.pitch_p;
-                CK(launch_field_sum(base + d.o_px + e, base + d.o_py + e, d.pitch_p, nr, d.nx, frame_buf.p + held, K.stream));
-                held += (size_t)nr * d.nx;
-                r += nr;
-            }
-        }
-        flush();
+        CK(cudaMemcpyAsync(q->frame.data(), dense, at * sizeof(float), cudaMemcpyDeviceToHost, K.stream));
+        CK(cudaStreamSynchronize(K.stream));
     }
 
     // info[4] = {active, queued, finished in this tick, steps advanced}.  The

@@ -307,3 +307,22 @@ def test_served_copy_jobs_follow_their_own_scene(monkeypatch, form):
         assert np.any(rec)
         assert rel(got[i][0], rec) <= 1e-6, (i, rel(got[i][0], rec))
         assert rel(got[i][1], frame) <= 1e-6, (i, rel(got[i][1], frame))
+
+
+def test_final_frames_take_no_device_memory():
+    """A final frame is summed in the finished scene's own memory: the device's
+    free memory is the same after a tick with one as after a tick without."""
+    import torch
+    from openpstd_gb300 import scenes
+    from openpstd_gb300.serving import Server
+    conf = scenes.plain_square(0, n=1500, steps=4, pml=50)
+    torch.cuda.mem_get_info()
+    with Server(512 << 20, max_scenes=2) as srv:
+        free = []
+        for flag in (False, True):
+            rid = srv.submit(conf, 2, final_frame=flag)
+            srv.run_until_idle(4)
+            _, frame = srv.result(rid)
+            free.append(torch.cuda.mem_get_info()[0])
+    assert frame.size == 1500 * 1500 and np.any(frame)
+    assert free[1] >= free[0]
