@@ -1144,9 +1144,10 @@ struct Kernel {
         steps = 0;
     }
 
+    int launches_per_stage() const { return chained ? 1 : (int)stage_launches().size(); }
     int launches_per_step() const {
         if (chained) return 7 + (spectral ? 2 : 0);
-        return 6 * (int)stage_launches().size() + (n_pml > 0 || dev_counts) + 1;
+        return 6 * launches_per_stage() + (n_pml > 0 || dev_counts) + 1;
     }
 
     // ---------------------------------------------------------------- chained form

@@ -538,7 +538,7 @@ int pstd_profile_passes(pstd_kernel* h, int32_t n_steps, void* stream, float* ms
         cudaEventDestroy(b);
         if (ms_stage) *ms_stage = ts;
         if (ms_total) *ms_total = tt;
-        if (stage_launches) *stage_launches = (int32_t)(n_steps * 6 * k->stage_launches().size());
+        if (stage_launches) *stage_launches = n_steps * 6 * k->launches_per_stage();
         if (total_launches) *total_launches = n_steps * k->launches_per_step();
         return PSTD_OK;
     })

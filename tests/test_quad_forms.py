@@ -94,3 +94,20 @@ def test_chained_receivers_and_steps(oracle_mod, monkeypatch, fam):
     assert np.array_equal(k.receivers(), want)
     assert all(np.array_equal(k.snapshot(i, "px"), p[i]) for i in range(k.domain_count()))
     assert rel(want, np.zeros_like(want)) > 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("env,chained", [({"PSTD_CHAIN": "0"}, True), ({"PSTD_AUTOTUNE": "0"}, False)])
+def test_profile_counts_the_launches_of_its_form(monkeypatch, env, chained):
+    from openpstd_gb300 import scenes
+    from openpstd_gb300.kernel import PSTDKernel
+    for k, v in env.items():
+        monkeypatch.setenv(k, v)
+    k = PSTDKernel()
+    k.initialize_kernel(scenes.l_shape(2, scale=0.2, steps=10))
+    lengths = k.plan_info().count("L=")
+    assert lengths >= 2
+    got = k.profile_passes(3)
+    assert got["stage_launches"] == 3 * 6 * (1 if chained else lengths)
+    assert got["total_launches"] == 3 * k.work_counts()["launches_per_step"] == got["stage_launches"] + 3 * (1 if chained else 2)
+    k.close()
