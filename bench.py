@@ -35,9 +35,9 @@ cell of a non-rigid domain advanced one step.
   speed of its own FFT set beside scipy's pocketfft on the same strip shapes
   (the reference links FFTW, which is absent here).
 
-``--impl reference`` times the reference's CPU algorithm (the oracle port; the
-reference itself cannot be built: Eigen, FFTW3f, Boost and Qt5 are absent) on
-the same scene with all host threads; under torchrun only rank 0 runs it.
+``--impl reference`` prints that the reference is unavailable: it cannot be
+built here (Eigen, FFTW3f, Boost and Qt5 are absent).  Its CPU algorithm,
+restated in oracle/, is timed as ``cpu_baseline``.
 Multi-GPU runs are replicas: every rank solves its own scene (seed = rank),
 no collective on the data path; value = all ranks' cells x steps / max time.
 """
@@ -486,41 +486,13 @@ def run_serve(args):
     print(json.dumps(line), flush=True)
 
 
-def run_reference(args):
-    # the reference's CPU path runs once, on rank 0; other ranks leave at once
-    # (no process group: nothing is exchanged)
-    rank, ws = int(os.environ.get("RANK", "0")), int(os.environ.get("WORLD_SIZE", "1"))
-    if rank != 0:
+def run_reference():
+    # the oracle port of its CPU path is timed as cpu_baseline, never in its place
+    if int(os.environ.get("RANK", "0")):
         return
-    from oracle import oracle
-    conf, desc = workload(args.workload, 0)
-    threads = os.cpu_count() or 1
-    # W warm-up steps are folded into one untimed step; K steps are timed,
-    # capped at ~90 s of host time (the rate is per step, so the cap only
-    # bounds the sample)
-    oracle.build()
-    s = oracle.OracleScene(conf, 32)
-    cells = sum(s.domain_info(i)["size"][0] * s.domain_info(i)["size"][1]
-                for i in range(s.n_domains) if not s.domain_info(i)["is_rigid"])
-    for _ in range(min(args.warmup, 1)):
-        s.run(1, threads=threads)
-    done, t0 = 0, time.perf_counter()
-    while done < args.steps:
-        s.run(1, threads=threads)
-        done += 1
-        if time.perf_counter() - t0 > 90:
-            break
-    el = time.perf_counter() - t0
-    v = cells * done / el / 1e9
-    line = {"metric": METRIC, "value": v, "unit": METRIC, "n_gpus": ws, "steps": done, "warmup": args.warmup,
-            "ms_per_step": el * 1e3 / done, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-            "dtype": "f32", "data": "synthetic (seeded scene)", "impl": "reference",
-            "config": {"workload": desc, "cells_per_step": cells, "steps_requested": args.steps},
-            "cpu_baseline": {"value": v, "unit": METRIC, "cores": threads, "kind": "port",
-                             "sample": f"{done} time steps of the workload (capped at 90 s)",
-                             "fft_speed": fft_speed(threads)},
-            "e2e": {"value": v, "unit": METRIC, "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0}}
-    print(json.dumps(line), flush=True)
+    print(json.dumps({"impl": "reference", "unavailable": "the reference cannot be built: Eigen, FFTW3f, Boost and Qt5 "
+                                                          "are absent, and its CMake lists missing kernel/DG sources"}),
+          flush=True)
 
 
 def run_ours(args):
@@ -700,7 +672,7 @@ def main():
     if args.warmup < 3:
         args.warmup = 3
     if args.impl == "reference":
-        run_reference(args)
+        run_reference()
     elif args.workload == "batch":
         run_batch(args)
     elif args.workload == "serve":
