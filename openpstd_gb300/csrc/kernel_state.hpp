@@ -130,8 +130,8 @@ inline bool gain_compensation() {
 
 // PSTD_PLAN="L:i,L:i,..." pins the variant of each listed strip length (for
 // profiling a plan the autotuner chose without a profiler); -1 = not listed.
-// PSTD_PLAN=serving pins every length to the plain variant with the
-// configuration of the serving loop's per-length persistent form.
+// PSTD_PLAN=serving pins every length to the variant with the configuration of
+// the serving loop's per-length persistent form.
 inline int planned_variant(int L) {
     const char* e = std::getenv("PSTD_PLAN");
     if (!e) return -1;

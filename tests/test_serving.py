@@ -326,3 +326,26 @@ def test_final_frames_take_no_device_memory():
             free.append(torch.cuda.mem_get_info()[0])
     assert frame.size == 1500 * 1500 and np.any(frame)
     assert free[1] >= free[0]
+
+
+@pytest.mark.parametrize("form", ["per_length", "merged", "lengths"])
+def test_copy_jobs_in_the_memory_of_an_earlier_scene(monkeypatch, form):
+    """Two scenes end together, so that the next one takes the second's slot in
+    the first's memory, full of its fields, while slot 0 holds a finished
+    scene: its copy jobs have to run by its own steps."""
+    from openpstd_gb300 import scenes
+    from test_plan_rules import _copying
+    from openpstd_gb300.serving import Server
+    _form_env(monkeypatch, form)
+    before = scenes.plain_square(0, n=150, steps=60, pml=50)
+    before.Speakers = [((10.25 + 20 * i) * 0.2, (10.25 + 20 * j) * 0.2, 0.0) for i in range(7) for j in range(7)]
+    conf = _copying(lr=("left", "right"))
+    with Server(256 << 20, max_scenes=8) as srv:
+        for c in (before, _copying(lr=())):
+            srv.submit(c, 20)
+        srv.run_until_idle(32)
+        rid = srv.submit(conf, 40, final_frame=True)
+        srv.run_until_idle(32)
+        rec, frame = srv.result(rid)
+    want_rec, want_frame = _solo(conf, 40)
+    assert rel(rec, want_rec) <= 1e-6 and rel(frame, want_frame) <= 1e-6, (rel(rec, want_rec), rel(frame, want_frame))
