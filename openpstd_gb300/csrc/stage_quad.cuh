@@ -23,11 +23,15 @@
 // domain, first-step flag, neighbour domain, data).  That chain, not the
 // arithmetic, is what a stage of a small scene spends its time on.
 //
-// Measured (GB300, one RK stage of a 96-scene batch, complex-strip form -> this
-// one, us): length 128 237 -> 169, 256 107 -> 73, 512 159 -> 117, 1024 174 ->
-// 139, 2048 52 -> 49; length 8192 of the 8192^2 scene 2822 -> 2360.  What bounds
-// it there: the L1 data path (66-75 % of its wavefronts; DRAM 27-35 %, issue
-// 36-44 %, ncu), i.e. the passes' trips through shared memory.
+// Measured (GB300, one RK stage of a 96-scene batch, fastest complex-strip
+// variant -> fastest of these, us): length 128 240 -> 172, 256 107 -> 73, 512
+// 160 -> 118, 1024 177 -> 139, 2048 53 -> 49; length 8192 of the 8192^2 scene
+// 2833 -> 2380.  (Length 128 took 163 as first built, with strips 0 and 2, 1 and
+// 3 sharing a transform; neighbours share one for their rounding.)  What bounds
+// lengths up to 1024 there: the L1 data path (69-76 % of its wavefronts; DRAM
+// 26-37 %, issue 44-49 %), i.e. the passes' trips through shared memory; about
+// 30 % of the shared load wavefronts are bank conflicts.  Counters:
+// profiles/stage_quad_batch.md.
 //
 // The kernels may be launched with programmatic stream serialisation: a CTA
 // reads its record and copies its tables before it waits for the previous
