@@ -1218,16 +1218,18 @@ struct Kernel {
         const DevJob* jobs;
         int n, tw_off, fp, fv, rc;
         bool all;
-        const int* cnt = nullptr;   // device-count persistent launch (launch_dev): its job count
+        const int* cnt = nullptr;   // device-count launch (launch_dev): its job count; n is its grid
         const QJob* qjobs = nullptr;   // four-strip form: its records
     };
-    // serving form, one persistent launch per strip length: the configuration,
-    // first job in djobs_all, index of the job count in dev_counts, twiddles
+    // serving form, one launch per strip length: the configuration, first job
+    // in djobs_all, index of the job count in dev_counts, twiddles, and the
+    // launch's grid (at least the job count)
     struct DevRegion {
         const StageVariant* var;
         size_t base;
         int count_idx;
         int tw_off;
+        int grid;
     };
     std::vector<DevRegion> dev_regions;
     struct SepBucket { int b, off, n; };
@@ -1252,7 +1254,7 @@ struct Kernel {
         if (dev_counts && !dev_regions.empty()) {
             for (size_t r = 0; r < dev_regions.size(); r++) {
                 const DevRegion& g = dev_regions[r];
-                StageLaunch l{g.var, djobs_all.p + g.base, 0, g.tw_off, 0, 0, 0, false};
+                StageLaunch l{g.var, djobs_all.p + g.base, g.grid, g.tw_off, 0, 0, 0, false};
                 l.cnt = dev_counts + g.count_idx;
                 l.qjobs = dqjobs_all.p + g.base;
                 v.push_back(l);
@@ -1499,7 +1501,7 @@ struct Kernel {
                 if (l.cnt) {
                     StageArgs a = stage_args(c, k, l.jobs, dtw.p + l.tw_off, 0, 0, 0);
                     a.qjobs = l.qjobs;
-                    CK(l.var->launch_dev(l.cnt, a, s));
+                    CK(l.var->launch_dev(l.cnt, l.n, a, s));
                 } else if (l.all && dev_counts) {
                     CK(launch_stage_all_dev(merged_fam, dev_counts, stage_args(c, k, l.jobs, dtw.p, 0, 0, 0),
                                             counters.p + k, s));

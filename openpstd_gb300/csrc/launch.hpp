@@ -75,11 +75,11 @@ struct StageVariant {
     cudaError_t (*prepare)();
     size_t (*smem_for)(int row_cap);                            // dynamic shared memory of one CTA
     const char* name;
-    // persistent form over a table of QJob records whose length is read from
-    // device memory at launch time (serving loop; null where not compiled):
-    // resident CTAs stride over it, skip all-zero entries and jobs of scenes at
-    // their step limit
-    cudaError_t (*launch_dev)(const int* count, const StageArgs& a, cudaStream_t st) = nullptr;
+    // over a table of QJob records whose length is read from device memory at
+    // launch time (serving loop; null where not compiled): one CTA per entry,
+    // grid >= length; all-zero entries and jobs of scenes at their step limit
+    // are skipped
+    cudaError_t (*launch_dev)(const int* count, int grid, const StageArgs& a, cudaStream_t st) = nullptr;
     cudaError_t (*prepare_dev)() = nullptr;
 };
 

@@ -210,7 +210,7 @@ struct Server {
     // arenas of entries, each scene's entries written once at admission and
     // zeroed at release.  Set 0 (one merged launch per stage): two regions,
     // transform length >= 1024 (taken first) and the rest with the copy jobs.
-    // Set 1 (one persistent launch per strip length): a region per length, a
+    // Set 1 (one launch per strip length): a region per length, a
     // scene's copy jobs in the region of its shortest length.  Counts in
     // device memory: {set 0: region 0 top, region 1 top, region 1 base; PML
     // domains, PML blocks, receivers, slots; set 1: top of region r at 7 + r}.
@@ -219,8 +219,10 @@ struct Server {
         const StageVariant* var = nullptr; // set 1: the configuration of the region's launch
         RangeAlloc a;
         size_t base = 0;                   // first entry in the job array
+        size_t grid = 0;                   // set 1: CTAs of the region's launch, one per entry in use and some ahead
     };
     static constexpr int MAX_REGIONS = 16;
+    static constexpr size_t GRID_MIN = 1024;   // (a launch's empty CTAs up to here take about a microsecond)
     bool pers_allowed = true, pers = false;
     int pset = 1;                          // configuration set of the persistent form
     RangeAlloc adom;
@@ -695,8 +697,18 @@ struct Server {
         moved |= put(drec, rec, 1 << 14);
         moved |= put(dslots, slots, (size_t)K.srv.n_flags);
         std::vector<Kernel::DevRegion> launches;
-        for (size_t r = 0; r < regs.size() && pset == 1; r++)
-            launches.push_back({regs[r].var, regs[r].base, 7 + (int)r, K.twiddles_of(regs[r].var)});
+        for (size_t r = 0; r < regs.size() && pset == 1; r++) {
+            // the grid is part of the captured graphs: it follows the entries in
+            // use by factors of two up (as the table grows) and eight down, as
+            // an entry past them costs a CTA that leaves at once
+            Region& g = regs[r];
+            const size_t top = g.a.top();
+            if (top > g.grid || (8 * top < g.grid && g.grid > GRID_MIN)) {
+                g.grid = std::min(g.a.cap, std::max(2 * top, GRID_MIN));
+                moved = true;
+            }
+            launches.push_back({g.var, g.base, 7 + (int)r, K.twiddles_of(g.var), (int)g.grid});
+        }
         if (K.filt.size() != filt_up) { moved |= put(K.dfilt, K.filt, 1 << 15); filt_up = K.filt.size(); }
         if (K.tw.size() != tw_up) { moved |= put(K.dtw, K.tw, 1 << 15); tw_up = K.tw.size(); }
         if (K.win.size() != win_up) { moved |= put(K.dwin, K.win, 1 << 13); win_up = K.win.size(); }

@@ -832,39 +832,30 @@ __global__ void __launch_bounds__(C::NT, C::MINB) stage_quad(const __grid_consta
     quad_job<C>(smq, A, J, A.tw, threadIdx.x);
 }
 
-// Serving loop: resident CTAs walk a record table whose length is read from
-// device memory, with a stride of the grid (records of one launch have one
-// length, so a job counter -- an atomic round trip and a barrier per job --
-// would balance little).  Free entries (all zero) and jobs of scenes that have
-// taken all their steps are skipped.
+// Serving loop: a record table whose length is read from device memory, one
+// CTA per entry of a grid that covers it; CTAs past the length, free entries
+// (all zero) and jobs of scenes that have taken all their steps leave at once.
+// As a loop over the table with resident CTAs the body spilled 0.2-1.3 KB a
+// thread (72-128 registers; called from the loop as a function, as much): 1500
+// resident scenes ran at 3.57 Gcell-steps/s, where the complex-strip loop before
+// it had made 3.94.  One job per CTA spills at most 144 bytes: 6.76.
 template <class C>
 __global__ void __launch_bounds__(C::NT, C::MINB) stage_quad_dev(const __grid_constant__ StageArgs A, const int* count) {
     extern __shared__ __align__(16) float4 smq[];
-    static_assert(!C::TSM, "the serving loop reads its tables through L1");
-    const int n = *count;
-    for (int j = blockIdx.x; j < n; j += gridDim.x) {
-        const QJob& J = A.qjobs[j];
-        const bool copy = J.kind & JK_COPY;
-        if ((J.L == 0 && !copy) || (A.scene_limit && A.scene_step[J.scene] >= A.scene_limit[J.scene])) continue;
-        if (copy) {
-            copy_axis<C::NT>(A, A.doms[J.dom], J.kind & JK_Y, threadIdx.x);
-            continue;
-        }
-        quad_body<C>(smq, A, J, A.tw, reinterpret_cast<const float4*>(A.filt + J.dtab), threadIdx.x);
-        __syncthreads();   // shared memory is the next job's
+    if ((int)blockIdx.x >= *count) return;
+    const QJob& J = A.qjobs[blockIdx.x];
+    const bool copy = J.kind & JK_COPY;
+    if ((J.L == 0 && !copy) || (A.scene_limit && A.scene_step[J.scene] >= A.scene_limit[J.scene])) return;
+    if (copy) {
+        copy_axis<C::NT>(A, A.doms[J.dom], J.kind & JK_Y, threadIdx.x);
+        return;
     }
+    quad_job<C>(smq, A, J, A.tw, threadIdx.x);
 }
 
 template <class C>
-cudaError_t launch_quad_dev_t(const int* count, const StageArgs& a, cudaStream_t st) {
-    static int grid = 0;
-    if (grid == 0) {
-        int dev, sms, per = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, stage_quad_dev<C>, C::NT, C::SMEM);
-        grid = sms * (per > 0 ? per : 1);
-    }
+cudaError_t launch_quad_dev_t(const int* count, int grid, const StageArgs& a, cudaStream_t st) {
+    if (grid <= 0) return cudaSuccess;
     stage_quad_dev<C><<<grid, C::NT, C::SMEM, st>>>(a, count);
     return cudaGetLastError();
 }

@@ -1,6 +1,6 @@
 // stage_serve.cu -- the stage kernel configurations of the serving loop's
-// per-length persistent form: one per transform length, each compiled with
-// the device-count persistent loop (stage_quad_dev).  They are the
+// per-length persistent form: one per transform length, each compiled as
+// the device-count kernel (stage_quad_dev).  They are the
 // configurations the autotuner picks on batches of scenes like the serving
 // stream (cells log-uniform 64x64 .. 1024x768, 50-cell PML), so a server
 // gets tuned arithmetic without timing variants on live scenes.  Each is also

@@ -349,3 +349,24 @@ def test_copy_jobs_in_the_memory_of_an_earlier_scene(monkeypatch, form):
         rec, frame = srv.result(rid)
     want_rec, want_frame = _solo(conf, 40)
     assert rel(rec, want_rec) <= 1e-6 and rel(frame, want_frame) <= 1e-6, (rel(rec, want_rec), rel(frame, want_frame))
+
+
+def test_launch_grids_follow_the_tables(monkeypatch):
+    """Forty scenes at once, then one: the per-length launches' grids grow with
+    the record tables and shrink again (one more capture), results as solo."""
+    from openpstd_gb300 import scenes
+    from openpstd_gb300.serving import Server
+    _form_env(monkeypatch, "lengths")
+    conf = scenes.plain_square(3, n=90, steps=30, pml=50)
+    want_rec, want_frame = _solo(conf, 20)
+    with Server(1 << 30, max_scenes=64) as srv:
+        ids = [srv.submit(conf, 20 if i == 39 else 2 + i % 3, final_frame=True) for i in range(40)]
+        srv.run_until_idle(32)
+        many = srv.result(ids[39])
+        grown = srv.stats()["graph_captures"]
+        rid = srv.submit(conf, 20, final_frame=True)
+        srv.run_until_idle(32)
+        one = srv.result(rid)
+        assert srv.stats()["graph_captures"] == grown + 1
+    for rec, frame in (many, one):
+        assert rel(rec, want_rec) <= 1e-6 and rel(frame, want_frame) <= 1e-6
