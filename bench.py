@@ -552,7 +552,7 @@ def run_ours(args):
     tpcs, tcase = traffic_per_cell_stage()
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                 "traffic": (tpcs * cells * 6 * prof_steps / launches) if tpcs else None,
-                "kernel": "stage_kernel<L,...> (all strip-length buckets of an RK stage)",
+                "kernel": "stage kernels (all strip-length buckets of an RK stage)",
                 "algorithmic_bytes_per_launch": alg_bytes / launches, "launches": launches,
                 "avg_launch_us": stage_ms * 1e3 / launches, "peak_source": f"{peak_kind} hbm_gbs",
                 "traffic_source": tcase, "stage_share_of_step": stage_ms / prof["ms_total"],
