@@ -685,6 +685,12 @@ struct Server {
             filt_up = tw_up = win_up = 0;
             moved = true;
         }
+        // a few entries left far out in a table that many scenes have filled:
+        // placed again from its start, so that the launches shrink to them
+        bool sparse = false;
+        for (const Region& g : regs) sparse |= pset == 1 && g.a.top() > GRID_MIN && g.a.top() > 4 * g.a.used;
+        for (Request* q : active)
+            if (sparse && q->placed) unplace(q);
         for (Request* q : active)
             if (!q->placed) moved |= place(q);
         std::vector<size_t> base;

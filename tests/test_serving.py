@@ -370,3 +370,25 @@ def test_launch_grids_follow_the_tables(monkeypatch):
         assert srv.stats()["graph_captures"] == grown + 1
     for rec, frame in (many, one):
         assert rel(rec, want_rec) <= 1e-6 and rel(frame, want_frame) <= 1e-6
+
+
+def test_a_scene_left_far_out_in_the_tables_moves(monkeypatch):
+    """Forty scenes, all but the last of them short: the one that goes on gets
+    its table entries written again from the tables' start, mid-solve."""
+    from openpstd_gb300 import scenes
+    from openpstd_gb300.serving import Server
+    _form_env(monkeypatch, "lengths")
+    conf, other = scenes.plain_square(3, n=90, steps=30, pml=50), scenes.l_shape(1, scale=0.1, steps=30)
+    with Server(1 << 30, max_scenes=64) as srv:
+        ids = [srv.submit(conf if i < 38 else other, 20 if i == 39 else 2 + i % 3, final_frame=True) for i in range(40)]
+        srv.tick(4)
+        assert srv.stats()["active"] == 1
+        grown = srv.stats()["graph_captures"]
+        srv.tick(5)
+        ids.append(srv.submit(conf, 20, final_frame=True))     # joins the moved scene
+        srv.run_until_idle(5)
+        assert srv.stats()["graph_captures"] == grown + 1
+        got = [srv.result(i) for i in ids[39:]]
+    for (rec, frame), c in zip(got, (other, conf)):
+        want_rec, want_frame = _solo(c, 20)
+        assert rel(rec, want_rec) <= 1e-6 and rel(frame, want_frame) <= 1e-6
